@@ -277,6 +277,7 @@ int prepare_points(knn_context* C, const void* points, int64_t n, int d, const k
 
 struct Trees {
   int32_t* perm = nullptr;
+  const int32_t* inv = nullptr;  // median trees: the inverse of each tree's order
   int depth = 0;
 };
 
@@ -307,6 +308,7 @@ int run_trees_segs(knn_context* C, const float* X, int64_t ntot, int d, int dpad
   rc = knn::tree_build(a, log);
   if (rc) return fail_cuda(cudaGetLastError(), "tree build launch");
   T->perm = a.perm;
+  T->inv = a.inv;
   T->depth = hsegs[0].depth;
   return KNN_OK;
 }
@@ -390,6 +392,7 @@ struct Layout {
   const int64_t* ftable = nullptr;
   const int64_t* foff = nullptr;
   const int64_t* fcount = nullptr;
+  const int32_t* tree_inv = nullptr;  // [trees][n] inverse orders of median trees
 };
 
 // Bound on the leaf blocks of a median tree of n points and this depth: node
@@ -512,7 +515,7 @@ int run_leaf_umma(knn_context* C, const float* X, int64_t n, int d, int dpad, in
                   int tc_group = 1) {
   const int kw = (k + 31) / 32;
   const int kq = k <= 16 ? 2 * k : 32;
-  const int Kp = ((d + 63) / 64) * 64;
+  const size_t ldr = (size_t)knn::umma_row_stride(d);
   knn::UmmaLeafArgs a{};
   a.X = X;
   a.n = n;
@@ -524,7 +527,6 @@ int run_leaf_umma(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   a.segs = lay.segs;
   a.leaves = lay.leaves;
   a.maxleaf = lay.maxleaf;
-  a.maxblock = lay.maxblock > 0 ? lay.maxblock : INT64_MAX;
   a.tc_group = std::min(std::max(tc_group, 1), lay.tc_group_max);
   a.ftable = lay.ftable;
   a.foff = lay.foff;
@@ -538,15 +540,20 @@ int run_leaf_umma(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   a.rkey = L->key[L->cur];
   a.rid = L->id[L->cur];
   a.f16 = precision == KNN_PREC_F16_RERANK;
-  int rc = C->get("Xb", (size_t)n * Kp * 2, &a.Xb);
+  int rc = C->get("Xb", (size_t)n * ldr * 2, &a.Xb);
+  if (!rc) rc = C->get("Xp", (size_t)n * ldr * 2, &a.Xp);
   if (!rc) rc = C->get("maxabs", 1, &a.maxabs);
   if (!rc) rc = C->get("norms2", (size_t)n, &a.norms2);
-  if (!rc && trees > 1) rc = C->get("linv", (size_t)n, &a.inv);
+  if (!rc) rc = C->get("norms_perm", (size_t)n, &a.np);
+  a.tree_inv = lay.tree_inv;
+  if (!rc && trees > 1 && !a.tree_inv) rc = C->get("linv", (size_t)n, &a.inv);
+  if (!rc && trees > 1) rc = C->get("plist", (size_t)n * kq, &a.plist);
+  const size_t srows = knn::umma_scratch_rows(a);
+  if (!rc) rc = C->get("survivors", srows * knn::umma_row_scratch_bytes(), &a.surv);
+  if (!rc) rc = C->get("surv_count", srows, &a.surv_count);
   if (!rc) rc = C->get("akey", (size_t)n * kq, &a.akey);
   if (!rc) rc = C->get("aid", (size_t)n * kq, &a.aid);
   if (rc) return rc;
-  knn::launch_init_lists(a.akey, a.aid, nullptr, n, kq, 1, st);
-  log.add();
   rc = knn::leaf_stage_umma(a, log);
   if (rc == KNN_ERR_UNSUPPORTED) return fail(rc, "tensor-core leaf stage: unsupported shape");
   if (rc) return fail_cuda(cudaGetLastError(), "tensor-core leaf stage launch");
@@ -972,6 +979,7 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
                            d <= 256 && k <= 32;
   Layout lay = single_layout(n, T.depth);
   lay.maxblock = host_max_block(n, T.depth, k);
+  lay.tree_inv = T.inv;
   {
     knn::SegEntry e{};
     e.n = n;
@@ -1185,6 +1193,7 @@ int group_compute(knn_context* C, const BatchGroup& g, int k, int trees, int pro
   lay.segs = view;
   lay.leaves = g.leaves;
   lay.maxleaf = g.maxleaf;
+  lay.tree_inv = T.inv;
   for (const auto& e : g.hsegs) lay.maxblock = std::max(lay.maxblock, host_max_block(e.n, e.depth, k));
   lay.tc_group_max = tc_group_max(g.hsegs.data(), (int)g.hsegs.size(), k, g.maxleaf);
   lay.own_blocks = leaves_own_blocks(g.hsegs.data(), (int)g.hsegs.size(), k);

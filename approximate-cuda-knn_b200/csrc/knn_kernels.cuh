@@ -136,17 +136,22 @@ struct UmmaLeafArgs {
   int d, dpad, k, kq, trees, metric;
   SegView segs;
   int64_t leaves, maxleaf;  // leaf blocks per tree; points in the largest leaf
-  int64_t maxblock;         // points in the largest leaf block (median trees)
   int tc_group;             // sibling leaves per 128-row tile: 1, 2 or 4 (each leaf its own block)
   const int32_t* perm;   // [trees][n]
   const float* norms;    // [n] FP32 norms (COSINE) or null
   bool f16;              // operands FP16 (else BF16)
-  void* Xb;              // [n][Kp] 16-bit operand scratch (Kp = d rounded up to 64)
+  void* Xb;              // [n][umma_row_stride(d)] 16-bit operand scratch
+  void* Xp;              // the same in a tree's order
   unsigned int* maxabs;  // [1] scratch: largest |x| (FP16 EUCLIDEAN row scale)
   float* norms2;         // [n] scratch
-  int32_t* inv;          // [n] scratch: a tree's inverse order (null: duplicate checks in the merge)
+  float* np;             // [n] scratch: norms2 in a tree's order
+  const int32_t* tree_inv;  // [trees][n] the trees' inverse orders, or null: computed into inv
+  int32_t* inv;          // [n] scratch (tree_inv null, several trees)
+  void* surv;            // [umma_scratch_rows(...)][umma_row_scratch_bytes()] scratch: the tiles' survivors
+  uint32_t* surv_count;  // [umma_scratch_rows(...)]
+  int32_t* plist;        // [n][kq] scratch: positions of the lists' entries (several trees)
   cudaEvent_t* kev;      // [2 * trees] events around each tree's tile kernel, or null
-  float* akey;           // [n][kq] approximate lists (in: empty)
+  uint32_t* akey;        // [n][kq] scratch: approximate lists (ordered keys and ids)
   uint32_t* aid;
   float* rkey;           // [n][k] out: exact keys, sorted
   uint32_t* rid;
@@ -157,6 +162,10 @@ struct UmmaLeafArgs {
   cudaStream_t stream;
 };
 int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log);
+size_t umma_scratch_rows(const UmmaLeafArgs& a);  // from the shape fields
+size_t umma_row_scratch_bytes();
+// Elements per row of the 16-bit operand copies: whole 16-byte units.
+inline int umma_row_stride(int d) { return (d + 7) & ~7; }
 
 struct PropArgs {
   const float* X;

@@ -13,22 +13,37 @@
 // coordinate and 2^24 per sum, e.g. the integer-mixture workload) the result
 // equals the FP32 leaf stage bit for bit.
 //
-// Tile: 128 queries x 128 candidates x Kp (Kp = d rounded up to 64, <= 256).
-//   * operands: K-major, 128-byte swizzled shared-memory tiles (8-row atoms of
-//     1024 B), filled by cp.async from the BF16 copy through the tree's order;
-//   * MMA: tcgen05.mma.cta_group::1.kind::f16, M=128 N=128 K=16, issued by one
-//     thread, accumulator 128 lanes x 128 columns of tensor memory, two
-//     accumulators so that one tile's MMA overlaps the previous tile's rounds;
-//   * completion: tcgen05.commit -> mbarrier, waited with an iteration limit
-//     (on expiry the block records an error, drains, frees TMEM and returns);
-//   * epilogue: per tile, tcgen05.ld 32x32b.x32 twice by all 8 warps (warp
-//     w reads lane quarter w%4, two 32-column slices); three instructions per
-//     key filter it against a slightly widened bound of the row's last entry
-//     into a survivor bit mask, then (while the next tile's MMA runs) the warps
-//     of each lane quarter read their rows' few survivors back from tensor
-//     memory, compute their exact keys and insert them into the query's sorted
-//     list (held in shared memory for the whole block) with one ballot and one
-//     lane shift each.  Two block barriers per tile.
+// Per tree the 16-bit rows are first copied into the tree's order
+// (k_permute_operand), so that a block's candidate tiles are plain 2-D boxes.
+// One thread block per (leaf, QT x 128 queries), warp-specialised:
+//   * a producer thread streams the block's candidates with TMA: boxes of 64
+//     rows x 64 elements (128-byte swizzle, 8 KB) into a ring;
+//   * an MMA thread issues tcgen05.mma.cta_group::1.kind::f16, M=128 N=64 K=16:
+//     the queries (A) stay in tensor memory for the whole block, the candidates
+//     (B) come from the ring, and QT query tiles share each candidate box; the
+//     FP32 accumulators rotate over NB 64-column buffers per query tile;
+//   * four epilogue warps per query tile, one per lane quarter: a thread owns a
+//     query row.  It reads a tile's two 32-column slices with tcgen05.ld
+//     32x32b.x32, filters the products against the row's bound into survivor
+//     bits, and appends the few survivors (product, column) to the row's buffer
+//     in an L2-resident scratch.
+// The stages meet only at mbarriers, so loads, products and filters of different
+// tiles overlap; no barrier spans the block between its prologue and end.
+// k_leaf_tc_merge then sorts each row's survivors and merges them into its list.
+//
+// What bounds it, and why this split.  The products of a 128 x 128 x 128 tile
+// take ~710 cycles of an SM's tensor pipe at the measured bf16 rate; the filter
+// needs two FP32 pipe and two ALU pipe cycles per 32 keys and scheduler, ~260-320
+// cycles.  Merging inside the tile kernel (a warp per survivor, two block barriers
+// per tile) held both to a few percent: 16 warps' latencies, and every warp waiting
+// for the slowest.  So the tile kernel only filters (16 epilogue warps per SM: two
+// blocks of two query tiles), and sorting runs at full occupancy in a kernel of
+// its own.  Integer mixture, 1M x 128, 8 trees, leaf 2048, k=16, tiles of all
+// trees: 30.8 ms with the in-kernel merge, 12.7 ms in this form (of which the merge
+// kernel 2.2 ms); 10M x 96 FP16 COSINE, 15 trees, leaf 4096: 431 -> 182 ms.  What
+// is left is the epilogue's latency chain (issue slots 50 % busy, tensor pipe
+// 28 % in the first tree).
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -40,35 +55,50 @@
 namespace knn {
 
 namespace {
-constexpr int kBM = 128;
-constexpr int kBN = 128;
-constexpr int kKC = 64;               // bf16 per 128-byte swizzled row
-constexpr int kChunkBytes = kBM * 128; // one 128 x 64 bf16 operand chunk
-constexpr uint32_t kTmemCols = 256;  // two 128-column accumulators
-constexpr int kUThreads = 256;
-constexpr int kRound = 64;          // tile columns per epilogue slice pair
-constexpr int kBulkMerge = 12;      // first tree: survivors in a 32-column slice from which sort + merge pays
+constexpr int kBM = 128;              // query rows of one accumulator
+constexpr int kTN = 64;               // candidate columns of one tile
+constexpr int kKC = 64;               // 16-bit elements per 128-byte swizzled row
+constexpr int kBoxBytes = kTN * 128;  // one 64 x 64 candidate box
+constexpr int kRing = 4;              // candidate boxes in flight (at least a tile's, four)
+// Survivors a row's buffer holds: rows of a later tree whose list is still poor
+// may see a hundred; 320 or 512 measured no faster (longer scratch rows).
+constexpr int kCap = 192;
+constexpr int kFlushAt = kCap - kTN;  // a fuller buffer could not take another tile
+constexpr int kFlushMin = 24;         // rows merged along when one row's buffer is full
+constexpr int64_t kChunkRows = 1 << 19;  // rows (of whole blocks) per launch: bounds the survivor scratch
+constexpr uint32_t kListed = 0x80000000u;  // count flag (first tree): the row's list was already written
+constexpr int kBand = 1024;           // block columns covered by the listed-column bitmap at a time
+constexpr int kBandWords = kBand / 32 + 1;
+constexpr int kNormSlots = 8;         // tiles of candidate norms staged ahead
+constexpr int kMergeRows = 4;         // rows merged together by a warp (independent chains)
+constexpr int kInsertMax = 5;         // candidates up to which one-by-one insertion beats sort and merge
+constexpr int kBoundRows = 4;         // the same for the bounding pass's selection
 constexpr float kSlack = 4.76837158203125e-07f;  // 2^-21: filter widening, eight units of FP32 rounding
-// Listed candidates inside the block, per row: sorted 16-bit column positions
-// ending in kXEnd (blocks of up to kXMaxBlock columns).
-constexpr int kXS = 33;
-constexpr uint32_t kXEnd = 0xFFFFu;
-constexpr int kXMaxBlock = 65000;
-// First tree: blocks of at least kPrepassMin columns get a bounding pass; its
-// group minima (64 per row, row stride kGS) use the list area.
+// Bounding pass: in the first kPrepassTrees trees, blocks of at least
+// kPrepassMin columns run their tiles once more beforehand; the group minima
+// (kGroups 32-column slices per row, wrapping, row stride kGS) overlay the
+// epilogue warp's shared memory.  In the second tree it replaces the tails of
+// rows whose first leaf was poor, which alone cost more than the pass: integer
+// mixture as above, tiles 14.9 -> 12.7 ms; a third tree's pass gains nothing.
+constexpr int kPrepassTrees = 2;
 constexpr int kPrepassMin = 1024;
 constexpr int kGroups = 64;
 constexpr int kGS = kGroups + 1;
-constexpr int kLS = 33;              // list row stride (row owners hit distinct banks)
-// A 128x128x256 tile finishes in about a microsecond; 2^16 polls with 32 ns
-// sleeps (a few ms) is far beyond that, and keeps a failing launch short.
-constexpr uint32_t kSpinLimit = 1u << 16;
+// Shared memory of one epilogue warp: a slice's products and the bitmaps of
+// listed columns (in the bounding pass: the group minima).
+constexpr int kDumpStride = 144;  // bytes of one row's 32 products, padded: 16-byte stores hit distinct banks
+constexpr int kWarpDump = 32 * kDumpStride;
+constexpr int kWarpBits = 32 * kBandWords * 4;
+constexpr int kWarpBytes = kWarpDump + kWarpBits;
+constexpr int kNormBytes = kNormSlots * (kTN + 4) * 4;  // -|y|^2 of a tile's columns, then the largest |y|^2
+static_assert(kWarpBytes >= 32 * kGS * 4, "group minima fit");
+static_assert(kWarpBytes % 16 == 0, "16-byte accesses");
 
 // Instruction descriptor of kind::f16: D f32 (bits 4-5 = 1), A and B format
 // at 7-9 and 10-12 (0 f16, 1 bf16; A and B always the same type), A and B
 // K-major (15, 16 = 0), N>>3 at 17-22, M>>4 at 24-28.
 constexpr uint32_t idesc_for(bool f16) {
-  return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((uint32_t)(kBN >> 3) << 17) |
+  return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((uint32_t)(kTN >> 3) << 17) |
          ((uint32_t)(kBM >> 4) << 24);
 }
 
@@ -92,49 +122,74 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int by
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
 }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
 
-// Non-blocking test of phase completion.  (try_wait may suspend the thread for
-// a system-dependent time per call, so counting try_wait calls bounds nothing;
-// test_wait never suspends.)
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+// Phase completion; may suspend the thread for at most about kPollNs.
+constexpr uint32_t kPollNs = 2000;
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}\n"
       : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      : "r"(bar), "r"(parity), "r"(kPollNs)
       : "memory");
   return ok != 0;
 }
 
 // Waits for the phase with the given parity; false once kWaitNs of wall time
-// (globaltimer) have passed.
-constexpr uint64_t kWaitNs = 20ull * 1000 * 1000;  // 20 ms; a tile takes ~1 us
+// (globaltimer) have passed, or once another wait of the block has given up.
+// The first to give up records it in the block's status and the error words:
+// err[0] stops the build's later blocks, err[1] stays until the host reports it.
+constexpr uint64_t kWaitNs = 20ull * 1000 * 1000;  // 20 ms; a tile takes under a microsecond
+constexpr uint32_t kSpinLimit = 1u << 20;
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* status, int* err) {
   const uint64_t t0 = global_ns();
   for (uint32_t it = 0; it < kSpinLimit; ++it) {
-    if (mbar_test_wait(bar, parity)) return true;
-    if (it > 64) {
-      __nanosleep(256);
-      if (global_ns() - t0 > kWaitNs) return false;
-    }
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*status != 0) return false;
+    if (global_ns() - t0 > kWaitNs) break;
   }
+  *status = 1;
+  atomicExch(err, 1);
+  atomicOr(err + 1, 1);
   return false;
 }
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* status, int* err) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_slow(bar, parity, status, err);
+}
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
-                                         uint32_t accumulate) {
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+// D (tensor memory) += A (tensor memory) x B (shared memory descriptor)
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc,
+                                            uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -142,13 +197,15 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
                : "memory");
 }
 
-__device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr) {
-  uint32_t v;
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(v) : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-  return v;
+__device__ __forceinline__ void tma_load_box(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::
+          "r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
 }
 
+// Issue only: the values are valid after tmem_wait_ld().
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -160,545 +217,762 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
         "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr));
+}
+// The loaded registers pass through the wait, so that no use of them can be
+// scheduled ahead of it.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(v[i]));
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]),
+      "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]),
+      "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
 }
 
-// Stage 128 gathered rows (ids in `ids`, <0: zero row) of the 16-bit copy
-// into a K-major 128B-swizzled operand of NCH 64-element chunks.  Thread t
-// always stages the same 16-byte unit (t mod 8 NCH) of rows t / (8 NCH) + i *
-// R, R = the rows one pass of the threads covers.
-template <int NCH>
-__device__ __forceinline__ void stage_operand(unsigned char* op, const uint16_t* __restrict__ Xb,
-                                              const int32_t* ids) {
-  constexpr int kUnitsPerRow = 8 * NCH;       // 16-byte units per row
-  constexpr int kRowsPerPass = kUThreads / kUnitsPerRow;
-  constexpr int kActive = kRowsPerPass * kUnitsPerRow;  // all 256 threads but for NCH = 3 (240)
-  const uint32_t base = smem_u32(op);
-  if (threadIdx.x < kActive) {
-    const int c16 = threadIdx.x % kUnitsPerRow;
-    const int chunk = c16 >> 3, w = c16 & 7;
-    const int r0 = threadIdx.x / kUnitsPerRow;
+// Two FP32 lanes in one instruction (each lane rounded as the scalar form).
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, uint32_t& lo, uint32_t& hi) {
+  asm("mov.b64 {%0, %1}, %2;\n" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// ------------------------------------------------------------- list merge --
+// Lists and candidates are (ordered key, id) pairs compared as one 64-bit
+// number: ordered keys are the FP32 keys mapped to integers of the same order.
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+__device__ __forceinline__ float from_orderable(uint32_t o) {
+  return __uint_as_float((o & 0x80000000u) ? (o ^ 0x80000000u) : ~o);
+}
+__device__ __forceinline__ bool pair_less(uint32_t ak, uint32_t ai, uint32_t bk, uint32_t bi) {
+  return (((uint64_t)ak << 32) | ai) < (((uint64_t)bk << 32) | bi);
+}
+
+// One compare-exchange step of R interleaved networks: lanes with keep_small
+// keep the smaller pair of themselves and lane ^ m.
+template <int R>
+__device__ __forceinline__ void exchange_rows(uint32_t (&k)[R], uint32_t (&id)[R], int m, bool keep_small) {
 #pragma unroll
-    for (int r = r0; r < kBM; r += kRowsPerPass) {
-      const uint32_t dst = base + chunk * kChunkBytes + r * 128 + ((w ^ (r & 7)) << 4);
-      const int32_t id = ids[r];
-      const uint16_t* src = Xb + (size_t)(id < 0 ? 0 : id) * (NCH * kKC) + c16 * 8;
-      cp_async16(dst, src, id < 0 ? 0 : 16);
+  for (int i = 0; i < R; ++i) {
+    const uint32_t ok = __shfl_xor_sync(0xFFFFFFFFu, k[i], m);
+    const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, id[i], m);
+    if (pair_less(ok, oi, k[i], id[i]) == keep_small) {
+      k[i] = ok;
+      id[i] = oi;
     }
   }
-  asm volatile("cp.async.commit_group;\n" ::);
 }
+// Equal pairs (two empty entries) may be exchanged either way: both are the same.
+
+// Ascending sort of the first `cnt` lanes (the others empty) of R rows: the
+// levels of the bitonic network up to the power of two that holds cnt.  The
+// steps are a loop: R rows keep the pipes busy, and straight-line code would not
+// stay in the instruction cache between merges.
+template <int R>
+__device__ __forceinline__ void sort_rows(uint32_t (&k)[R], uint32_t (&id)[R], int cnt) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int size = 2; size <= 32 && (size >> 1) < cnt; size <<= 1) {  // warp-uniform
+#pragma unroll 1
+    for (int m = size >> 1; m >= 1; m >>= 1)
+      exchange_rows<R>(k, id, m, ((lane & size) == 0) == ((lane & m) == 0));
+  }
+}
+
+// The candidates of the first `cnt` lanes one by one into R sorted lists: the
+// lanes whose entry is greater form a suffix, which shifts up one lane (the last
+// entry drops out).  An empty candidate is greater than every entry.
+template <int R>
+__device__ __forceinline__ void insert_rows(uint32_t (&lk)[R], uint32_t (&li)[R], const uint32_t (&ck)[R],
+                                            const uint32_t (&ci)[R], int cnt) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int e = 0; e < cnt; ++e) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const uint32_t k1 = __shfl_sync(0xFFFFFFFFu, ck[i], e), i1 = __shfl_sync(0xFFFFFFFFu, ci[i], e);
+      const uint32_t uk = __shfl_up_sync(0xFFFFFFFFu, lk[i], 1), ui = __shfl_up_sync(0xFFFFFFFFu, li[i], 1);
+      const bool after = pair_less(k1, i1, lk[i], li[i]);
+      const bool before = lane == 0 || !pair_less(k1, i1, uk, ui);  // the entry below stays
+      if (after) {
+        lk[i] = before ? k1 : uk;
+        li[i] = before ? i1 : ui;
+      }
+    }
+  }
+}
+
+// Lists <- the 32 smallest of list and sorted candidates.
+template <int R>
+__device__ __forceinline__ void merge_lower_rows(uint32_t (&lk)[R], uint32_t (&li)[R], const uint32_t (&ck)[R],
+                                                 const uint32_t (&ci)[R]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const uint32_t rk = __shfl_sync(0xFFFFFFFFu, ck[i], 31 - lane);
+    const uint32_t ri = __shfl_sync(0xFFFFFFFFu, ci[i], 31 - lane);
+    if (pair_less(rk, ri, lk[i], li[i])) {  // min(list, reversed candidates) is bitonic
+      lk[i] = rk;
+      li[i] = ri;
+    }
+  }
+#pragma unroll 1
+  for (int m = 16; m >= 1; m >>= 1) exchange_rows<R>(lk, li, m, (lane & m) == 0);
+}
+
+// Tensor-memory columns of a block: QT * NB accumulators, then QT query tiles.
+// Up to 128 dims a block takes 128 columns per query tile, else 256.
+template <int NCH, int QT>
+struct TmemPlan {
+  static constexpr int kTotal = NCH <= 2 ? 128 * QT : 256;
+  static constexpr int kA = NCH * 32;                              // columns of one query tile
+  static constexpr int kNB = (kTotal - QT * kA) / (QT * kTN);      // accumulators per query tile
+  static constexpr int kA0 = QT * kNB * kTN;
+  static constexpr int kBlocks = NCH <= 2 && QT == 1 ? 3 : 2;      // resident blocks per SM
+  static_assert(kNB >= 1 && kA0 + QT * kA <= kTotal && kBlocks * kTotal <= 512, "tensor memory plan");
+};
 
 }  // namespace
 
-// Ascending sort of one value per lane (bitonic network over the warp).
-__device__ __forceinline__ uint32_t warp_sort32_u32(uint32_t v) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-    for (int m = size >> 1; m >= 1; m >>= 1) {
-      const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v, m);
-      const bool keep_min = ((lane & size) == 0) == ((lane & m) == 0);
-      v = keep_min ? min(v, o) : max(v, o);
-    }
-  }
-  return v;
-}
+struct LeafTcArgs {
+  const uint16_t* Xp;     // [n][ldr] 16-bit rows in the tree's order
+  const float* np;        // [n] their norms in the tree's order (EUCLIDEAN)
+  const int32_t* perm;    // [n] the tree's order
+  const int32_t* plist;   // [n][kq] later trees: the position of every list entry, rows in the tree's order
+  const int64_t* ftab;    // leaf table (reference-rule trees) or null
+  SegView segs;
+  uint32_t* akey;         // [n][kq] ordered keys
+  uint32_t* aid;          // [n][kq]
+  uint2* surv;            // [blocks of the launch][128 QT][kCap] survivors: product, block column
+  uint32_t* count;        // [blocks of the launch][128 QT] survivors of each row, kListed
+  int64_t block0;         // first block of the launch
+  int* err;
+  int64_t n;
+  uint32_t idesc;
+  int ldr, ksteps;        // row stride in elements; 16-element steps holding dims
+  int k, kq, qtiles, glog;
+};
 
-// One block per (leaf, 128-query tile), stepping over the block's 128-column
-// candidate tiles.  The 128 queries' lists stay in shared memory for the whole
-// block (read once, written once).  Each step empties one 128x128 tensor-core
-// tile (tensor memory, two 128-column buffers):
-//   * epilogue: thread (row, 32-column half) loads the products of its two
-//     32-column slices (tcgen05.ld 32x32b.x32), filters them against a
-//     conservative bound of the row's list tail at the step's start into
-//     survivor bit masks (three instructions per key), drops the row's own
-//     column and listed ids;
-//   * merge: the warps of the rows' lane quarter insert each row's survivors,
-//     reading their products back from tensor memory (tcgen05.ld x1 per
-//     survivor, or x32 and a lane transpose for a bulk batch), computing the
-//     exact keys and applying the exact (key, id) rule.
-// The next step's operand is staged while the epilogue runs (its MMA has
-// completed), and its MMA runs into the other tensor-memory buffer during
-// the merge.  MMA issue, bounded waits and the tensor-memory loads follow the
-// single-tile sequence that was checked on its own against a CPU product.
-// FIRST: the launch of the first tree, whose lists start empty; a point then
-// meets every candidate once, so no survivor can already be listed, and a
-// 32-column slice with many survivors is sorted and merged into the list in one go.
-// Blocks of kPrepassMin columns or more first run all tiles once (pass 0) to
-// record each row's smallest exact key in each of kGroups column groups
-// (32-column slices, wrapping); the kq-th smallest group minimum is the key of
-// kq distinct candidates, so it bounds the kq-th key of the final list, and
-// pass 1 filters against it from its first tile on.
-// Later trees, with inv (the tree's inverse order): the block's columns that
-// hold an id already in the row's list are found up front (inv of each listed
-// id) and masked out of the survivors, so the merge needs no duplicate check;
-// a candidate meets a row once per tree, so ids inserted during the block
-// cannot come back.
-template <int METRIC, bool FIRST, int NCH>
-__global__ void __launch_bounds__(kUThreads, 2)
-    k_leaf_tc(const uint16_t* __restrict__ Xb, uint32_t idesc, SegView segs,
-              const int64_t* __restrict__ ftab, int k, int kq,
-              int qtiles, int glog, const int32_t* __restrict__ perm, const int32_t* __restrict__ inv,
-              const float* __restrict__ norms2, float* __restrict__ akey, uint32_t* __restrict__ aid,
-              int* __restrict__ err) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int nchunks = NCH;
-  unsigned char* opA = smem;
-  unsigned char* opB = opA + nchunks * kChunkBytes;
-  float* Lk = reinterpret_cast<float*>(opB + nchunks * kChunkBytes);  // [128][kLS] list keys
-  uint32_t* Li = reinterpret_cast<uint32_t*>(Lk + kBM * kLS);         // [128][kLS] list ids
-  int32_t* qid = reinterpret_cast<int32_t*>(Li + kBM * kLS);
-  float* qn = reinterpret_cast<float*>(qid + kBM);
-  int32_t* cid3 = reinterpret_cast<int32_t*>(qn + kBM);  // [3][128] candidate ids, slot = step mod 3
-  float* cn3 = reinterpret_cast<float*>(cid3 + 3 * kBN);  // [3][128] norms (EUCLIDEAN) or 0; +inf: padding
-  uint32_t* msk = reinterpret_cast<uint32_t*>(cn3 + 3 * kBN);  // [128][4] survivor bits of the step's tile
-  float* cmax3 = reinterpret_cast<float*>(msk + kBM * 4);      // [3][4] largest candidate norm per warp
-  uint16_t* xp = reinterpret_cast<uint16_t*>(cmax3 + 12);      // [128][kXS] listed columns
-  float* tcap = reinterpret_cast<float*>(xp + kBM * kXS);      // [128] first tree: bound on the kq-th key
-  // [128][2] grouped leaves: the row's own columns (in the listed-column area,
-  // unused then: a grouped tile is one column tile, so xcl is off)
-  int16_t* rcol = reinterpret_cast<int16_t*>(xp);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(tcap + kBM);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 1);
-  int* status = reinterpret_cast<int*>(tmem_slot + 1);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t leaf = blockIdx.x / qtiles;
-  const int qt = (int)(blockIdx.x - leaf * qtiles);
-  int64_t lo, hi, blo, bhi;
-  if (ftab) {  // explicit leaf table (reference-rule trees)
-    const int64_t* e = ftab + 4 * leaf;
-    lo = e[0];
-    hi = e[1];
-    blo = e[2];
-    bhi = e[3];
-  } else if (glog == 0) {
-    int64_t j;
-    const SegEntry seg = segs.leaf(leaf, &j);
-    leaf_block(seg, j, k, &lo, &hi, &blo, &bhi);
+// Block b's leaf rows [lo, hi), candidate block [blo, bhi) (positions in the
+// tree's order) and first query row q0 of the leaf.
+struct BlockRange {
+  int64_t lo, hi, blo, bhi, j;
+  SegEntry seg;
+  int q0;
+};
+template <int QT>
+__device__ __forceinline__ BlockRange block_range(const LeafTcArgs& a, int64_t b) {
+  BlockRange g{};
+  const int64_t leaf = b / a.qtiles;
+  g.q0 = (int)(b - leaf * a.qtiles) * (kBM * QT);
+  if (a.ftab) {  // explicit leaf table (reference-rule trees)
+    const int64_t* e = a.ftab + 4 * leaf;
+    g.lo = e[0];
+    g.hi = e[1];
+    g.blo = e[2];
+    g.bhi = e[3];
+  } else if (a.glog == 0) {
+    g.seg = a.segs.leaf(leaf, &g.j);
+    leaf_block(g.seg, g.j, a.k, &g.lo, &g.hi, &g.blo, &g.bhi);
   } else {
     // 2^glog sibling leaves, each its own block (the host checks that every
     // leaf holds k+1 points), as one tile: a row keeps only its own leaf's
-    // columns (rcol)
-    int64_t j;
-    const SegEntry seg = segs.leaf(leaf << glog, &j);
-    lo = blo = seg.off + node_lo(seg.n, seg.depth, j);
-    hi = bhi = seg.off + node_lo(seg.n, seg.depth, j + (int64_t(1) << glog));
-    if (threadIdx.x < kBM) {
-      const int64_t p = lo + threadIdx.x;
-      int64_t a = lo, b = lo;
-      for (int g = 0; g < (1 << glog); ++g) {
-        const int64_t e = seg.off + node_lo(seg.n, seg.depth, j + g + 1);
-        if (p < e) {
-          b = e;
-          break;
-        }
-        a = e;
+    // columns
+    g.seg = a.segs.leaf(leaf << a.glog, &g.j);
+    g.lo = g.blo = g.seg.off + node_lo(g.seg.n, g.seg.depth, g.j);
+    g.hi = g.bhi = g.seg.off + node_lo(g.seg.n, g.seg.depth, g.j + (int64_t(1) << a.glog));
+  }
+  return g;
+}
+
+// Merge the buffered survivors of the rows in `rows` (warp-uniform) into their
+// lists, kMergeRows rows at a time: every row's loads, sort and merge are
+// independent chains.  Lane r holds row r's id, norm, count and bound; surv the
+// rows' buffers (product, block column); np and perm start at the block.  Returns the
+// bounds, lowered to the new list tails.
+template <int METRIC>
+__device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, const float* np, const int32_t* perm,
+                                                 int kq, const uint2* surv, int qid, float myn, int cnt, float tk,
+                                                 uint32_t have, uint32_t rows) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  while (rows) {
+    uint32_t lk[kMergeRows], li[kMergeRows], ck[kMergeRows], ci[kMergeRows];
+    int r[kMergeRows], c[kMergeRows];
+    int most = 0;
+    bool fresh = true;  // warp-uniform
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) {  // fewer rows left: the last one again (same result)
+      r[i] = rows ? __ffs(rows) - 1 : r[i > 0 ? i - 1 : 0];
+      rows &= rows - 1;
+    }
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) {
+      const int id = __shfl_sync(0xFFFFFFFFu, qid, r[i]);
+      c[i] = __shfl_sync(0xFFFFFFFFu, cnt, r[i]);
+      most = max(most, c[i]);
+      lk[i] = kNoKey;
+      li[i] = kNoId;
+      fresh = fresh && !((have >> r[i]) & 1u);
+      if (lane < kq && ((have >> r[i]) & 1u)) {
+        lk[i] = akey[(size_t)id * kq + lane];
+        li[i] = aid[(size_t)id * kq + lane];
       }
-      rcol[2 * threadIdx.x] = (int16_t)(a - blo);
-      rcol[2 * threadIdx.x + 1] = (int16_t)(b - blo);
+    }
+    for (int e0 = 0; e0 < most; e0 += 32) {
+#pragma unroll
+      for (int i = 0; i < kMergeRows; ++i) {
+        const float xn = __shfl_sync(0xFFFFFFFFu, myn, r[i]);
+        ck[i] = kNoKey;
+        ci[i] = kNoId;
+        if (e0 + lane < c[i]) {
+          const uint2 v = surv[r[i] * kCap + e0 + lane];
+          const float dot = __uint_as_float(v.x);
+          const uint32_t p = v.y;
+          ck[i] = orderable(METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(xn, np[p]))
+                                                           : __fsub_rn(1.f, dot));
+          ci[i] = (uint32_t)perm[p];
+        }
+      }
+      if (most - e0 <= kInsertMax) {
+        insert_rows<kMergeRows>(lk, li, ck, ci, most - e0);
+        continue;
+      }
+      sort_rows<kMergeRows>(ck, ci, most - e0);
+      if (fresh && e0 == 0) {  // empty lists: the sorted candidates are the lists
+#pragma unroll
+        for (int i = 0; i < kMergeRows; ++i) {
+          lk[i] = ck[i];
+          li[i] = ci[i];
+        }
+      } else {
+        merge_lower_rows<kMergeRows>(lk, li, ck, ci);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) {
+      const int id = __shfl_sync(0xFFFFFFFFu, qid, r[i]);
+      if (lane < kq) {
+        akey[(size_t)id * kq + lane] = lk[i];
+        aid[(size_t)id * kq + lane] = li[i];
+      }
+      const float tail = from_orderable(__shfl_sync(0xFFFFFFFFu, lk[i], kq - 1));
+      if (lane == r[i] && tail < tk) tk = tail;  // NaN: an empty slot
     }
   }
-  const int nq = (int)(hi - lo);
-  const int q0 = qt * kBM;
-  if (q0 >= nq) return;  // whole block, before any barrier or allocation
-  const int mq = min(kBM, nq - q0);
-  const int nb = (int)(bhi - blo);
-  const int ntiles = (nb + kBN - 1) / kBN;
-  // Listed ids are located up front only in blocks of several tiles: in a
-  // one-tile block the few survivors are cheaper to check by the merge's ballot.
-  const bool xcl = !FIRST && inv != nullptr && nb > kBN && nb <= kXMaxBlock;  // block-uniform
-  const bool pre = FIRST && nb >= kPrepassMin && glog == 0;
-  const int nsteps = pre ? 2 * ntiles : ntiles;
-  const float kInf = __int_as_float(0x7F800000);
-  const float kMaxF = __int_as_float(0x7F7FFFFF);
-  const uint32_t bar = smem_u32(mbar);
-  float* gm = Lk;  // [128][kGS] group minima during pass 0 (spans Lk and Li)
+  __syncwarp();
+  return tk;
+}
 
-  if (warp == 0) {
+// One block per (leaf, QT x 128 queries).  FIRST: the launch of the first
+// tree, whose lists start empty and are all written.  PRE: blocks of
+// kPrepassMin columns or more run their tiles twice: pass 0 records each row's
+// smallest key' (below) in each of kGroups column groups; the kq-th smallest
+// group minimum belongs to kq distinct candidates, so, widened by the rounding
+// of key' against the exact key, it bounds the kq-th key of the list after this
+// tree, and pass 1 filters against it from its first tile on.
+// Later trees: the block's columns that hold an id already in a row's list
+// (k_list_positions) are kept as a bitmap, kBand columns at a time, and masked
+// out of the survivors, so a candidate meets a list at most once and merging
+// needs no duplicate check.
+// Row filter, a superset of what the exact rule (key <= the row's list tail
+// tk) can admit: key' = |y|^2 - 2 x.y (EUCLIDEAN) or -x.y (COSINE) against
+// thr = tk - |x|^2 (or tk - 1) widened by 2^-21 (|tk| + |x|^2 + max|y|^2),
+// which bounds the rounding of both the key and the threshold.  A tail from an
+// earlier tile is looser than the current one, never tighter.  Every
+// survivor's exact key is computed at its merge and ranked there.
+template <int METRIC, bool FIRST, bool PRE, int NCH, int QT>
+__global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
+    k_leaf_tc(const __grid_constant__ CUtensorMap bmap, const __grid_constant__ LeafTcArgs a) {
+  using Plan = TmemPlan<NCH, QT>;
+  constexpr int NB = Plan::kNB, RING = kRing;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* ring = smem;
+  unsigned char* warp_area = ring + RING * kBoxBytes;
+  float* tnorms = reinterpret_cast<float*>(warp_area + 4 * QT * kWarpBytes);  // [kNormSlots][kTN + 4]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(tnorms) + kNormBytes);
+  // ring full [RING], ring empty [RING], accumulators full [QT][NB], empty [QT][NB], norms full, empty, drained
+  const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * RING;
+  const uint32_t bar_afull = bar_empty + 8 * RING, bar_aempty = bar_afull + 8 * QT * NB;
+  const uint32_t bar_nfull = bar_aempty + 8 * QT * NB, bar_nempty = bar_nfull + 8 * kNormSlots;
+  const uint32_t bar_done = bar_nempty + 8 * kNormSlots;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * RING + 2 * QT * NB + 2 * kNormSlots + 1);
+  int* status_p = reinterpret_cast<int*>(tmem_slot + 1);
+  volatile int* status = status_p;
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);  // warp-uniform
+  const BlockRange range = block_range<QT>(a, a.block0 + blockIdx.x);
+  const int64_t lo = range.lo, blo = range.blo, bhi = range.bhi;
+  const int nq = (int)(range.hi - lo), q0 = range.q0;
+  if (q0 >= nq) return;  // whole block, before any barrier or allocation
+  const int nb = (int)(bhi - blo);
+  const int qts = min(QT, (nq - q0 + kBM - 1) / kBM);  // query tiles with rows
+  const int nt = (nb + kTN - 1) / kTN;
+  const int npre = PRE && nb >= kPrepassMin && a.glog == 0 ? nt : 0;  // tiles of the bounding pass
+  const int nsteps = npre + nt;
+
+  if (warp == 4 * QT) {  // producer warp: barriers
     if (lane == 0) {
-      mbar_init(bar, 1);
+      for (int i = 0; i < RING; ++i) {
+        mbar_init(bar_full + 8 * i, 1);
+        mbar_init(bar_empty + 8 * i, 1);
+      }
+      for (int i = 0; i < QT * NB; ++i) {
+        mbar_init(bar_afull + 8 * i, 1);
+        mbar_init(bar_aempty + 8 * i, 4);
+      }
+      for (int i = 0; i < kNormSlots; ++i) {
+        mbar_init(bar_nfull + 8 * i, 1);
+        mbar_init(bar_nempty + 8 * i, 4 * qts);
+      }
+      mbar_init(bar_done, 1);
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-      *status = 0;
+      // an earlier block of the build gave up: do nothing
+      *status_p = *reinterpret_cast<volatile int*>(a.err) != 0 ? 2 : 0;
     }
     __syncwarp();
+  } else if (warp == 4 * QT + 1) {  // MMA warp: tensor memory
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kTmemCols));
+                 "r"((uint32_t)Plan::kTotal));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
-  if (tid < kBM) {
-    const int32_t id = tid < mq ? perm[lo + q0 + tid] : -1;
-    qid[tid] = id;
-    qn[tid] = (METRIC == KNN_METRIC_EUCLIDEAN && id >= 0) ? norms2[id] : 0.f;
-    tcap[tid] = kInf;
-  }
-  // candidates of step s (warps 0-3, whole warps) into slot s mod 3;
-  // fetch_cols loads them into registers (a step ahead), put_cols stores them
-  int32_t nid = -1;
-  float nnv = 0.f;
-  auto fetch_cols = [&](int s) {
-    const int c0 = (s % ntiles) * kBN, mc = min(kBN, nb - c0);
-    nid = tid < mc ? perm[blo + c0 + tid] : -1;
-    nnv = (METRIC == KNN_METRIC_EUCLIDEAN && nid >= 0) ? norms2[nid] : 0.f;
-  };
-  auto put_cols = [&](int s) {
-    cid3[(s % 3) * kBN + tid] = nid;
-    cn3[(s % 3) * kBN + tid] = nid >= 0 ? nnv : kInf;
-    // norms are >= 0, so their bit patterns order as unsigned integers
-    const uint32_t wm = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(nnv));
-    if (lane == 0) cmax3[(s % 3) * 4 + warp] = __uint_as_float(wm);
-  };
-  if (tid < kBN) {
-    fetch_cols(0);
-    put_cols(0);
-    if (nsteps > 1) fetch_cols(1);
-  }
-  __syncthreads();
-  stage_operand<NCH>(opA, Xb, qid);
-  stage_operand<NCH>(opB, Xb, cid3);
-  if (pre) {
-    for (int e = tid; e < kBM * kGS; e += kUThreads) gm[e] = kInf;
-  } else {
-    // warp w: rows w + 8 i, lane s: entry s; all loads issued before use
-    float lkr[kBM / 8];
-    uint32_t lir[kBM / 8];
-#pragma unroll
-    for (int i = 0; i < kBM / 8; ++i) {
-      const int32_t id = qid[warp + 8 * i];
-      const bool live = id >= 0 && lane < kq;
-      lkr[i] = live ? akey[(size_t)id * kq + lane] : kInf;
-      lir[i] = live ? aid[(size_t)id * kq + lane] : kNoId;
-    }
-#pragma unroll
-    for (int i = 0; i < kBM / 8; ++i) {
-      Lk[(warp + 8 * i) * kLS + lane] = lkr[i];
-      Li[(warp + 8 * i) * kLS + lane] = lir[i];
-    }
-    if (xcl) {
-      // the listed ids' columns in this block, sorted per row: the 16 rows'
-      // bitonic networks interleaved stage by stage, two rows' 16-bit
-      // positions packed per register (halfword min / max)
-      uint32_t pk[kBM / 16];
-#pragma unroll
-      for (int i = 0; i < kBM / 8; ++i) {
-        uint32_t p = kXEnd;
-        if (lir[i] != kNoId) {
-          const int64_t q = (int64_t)inv[lir[i]] - blo;
-          if (q >= 0 && q < nb) p = (uint32_t)q;
-        }
-        if (i & 1) pk[i >> 1] |= p << 16;
-        else pk[i >> 1] = p;
-      }
-#pragma unroll
-      for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-        for (int m = size >> 1; m >= 1; m >>= 1) {
-          const bool keep_min = ((lane & size) == 0) == ((lane & m) == 0);
-#pragma unroll
-          for (int j = 0; j < kBM / 16; ++j) {
-            const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, pk[j], m);
-            pk[j] = keep_min ? __vminu2(pk[j], o) : __vmaxu2(pk[j], o);
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < kBM / 8; ++i) {
-        xp[(warp + 8 * i) * kXS + lane] = (uint16_t)((i & 1) ? (pk[i >> 1] >> 16) : (pk[i >> 1] & 0xFFFFu));
-        if (lane == 0) xp[(warp + 8 * i) * kXS + 32] = (uint16_t)kXEnd;
-      }
-    }
-  }
-  int xptr = 0;  // this thread's next entry of its row's listed columns
-
-  // step 0's MMA
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  auto issue_mma = [&](int s) {  // thread 0: operands staged, previous MMA waited for
-    if (*reinterpret_cast<volatile int*>(err) != 0) {
-      *status = 2;  // another block failed: issue nothing more
-      return;
-    }
-    const uint32_t a0 = smem_u32(opA), b0 = smem_u32(opB);
-    const uint32_t d = tmem + (uint32_t)((s & 1) * kBN);
-    for (int ch = 0; ch < nchunks; ++ch)
-#pragma unroll
-      for (int kk = 0; kk < kKC / 16; ++kk) {
-        const uint32_t off = ch * kChunkBytes + kk * 32;
-        umma_f16(d, desc_sw128(a0 + off), desc_sw128(b0 + off), idesc, (ch | kk) != 0 ? 1u : 0u);
-      }
-    umma_commit(bar);
-  };
-  if (tid == 0) issue_mma(0);
+  const bool stopped = *status != 0;  // block-uniform: read after the barrier, not written before the next
 
-  // Per step: [A] MMA(s) done -> stage B(s+1) -> epilogue over the tile's 128
-  // columns (two 32-column slices per thread) -> [B] -> MMA(s+1) issued ->
-  // merge of the step's survivors -> the next step's [A].  Candidate ids and
-  // norms live in three slots (step s in slot s mod 3): the merge of step s
-  // still reads its slot while step s+1 fills slot (s+2) mod 3.
-  uint32_t phase = 0;
-  for (int s = 0; s < nsteps; ++s) {
-    const int pass = pre && s < ntiles ? 0 : 1;
-    const int c0 = (s % ntiles) * kBN, mc = min(kBN, nb - c0);
-    const bool has_next = s + 1 < nsteps;
-    if (has_next && tid < kBN) {
-      put_cols(s + 1);
-      if (s + 2 < nsteps) fetch_cols(s + 2);
-    }
-    if (tid == 0 && *status == 0 && !mbar_wait_bounded(bar, phase)) {
-      *status = 1;
-      atomicExch(err, 1);     // this build's blocks stop issuing MMAs
-      atomicOr(err + 1, 1);   // sticky until the host reports it
-      mbar_wait_bounded(bar, phase);  // let the MMAs drain before TMEM is freed
-    }
-    phase ^= 1u;
-    __syncthreads();  // [A]
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (*status != 0) break;  // uniform: read after the barrier
-    // step s's MMA has completed: B is free for step s + 1
-    if (has_next) stage_operand<NCH>(opB, Xb, cid3 + ((s + 1) % 3) * kBN);
-    const int32_t* cid = cid3 + (s % 3) * kBN;
-    const float* cn = cn3 + (s % 3) * kBN;
-    const float* cmx = cmax3 + (s % 3) * 4;
-    const float cm = fmaxf(fmaxf(cmx[0], cmx[1]), fmaxf(cmx[2], cmx[3]));
-    const uint32_t tbuf = tmem + (uint32_t)((s & 1) * kBN);
-    const int quarter = warp & 3, half = warp >> 2;
-    const uint32_t tq = tbuf + ((uint32_t)(quarter * 32) << 16);  // this warp's lane quarter
-    const int r = quarter * 32 + lane;
-    // the row's filter bound (pass 1), from its list tail at the step's start
-    float thr = 0.f;
-    if (pass == 1) {
-      // Row filter, a superset of what the exact rule (key <= the row's
-      // list tail tk) can admit: key' = |y|^2 - 2 x.y (EUCLIDEAN) or
-      // -x.y (COSINE) against thr = tk - |x|^2 (or tk - 1) widened by
-      // 2^-21 (|tk| + |x|^2 + max|y|^2), which bounds the rounding of
-      // both the key and the threshold.  Padding columns have key' =
-      // +inf, a row outside the block thr = -inf, a list with free slots
-      // thr = FLT_MAX.  A bound from the step's start is looser than the
-      // current tail, never tighter, so the filter stays a superset.
-      const float tk = FIRST ? fminf(Lk[r * kLS + kq - 1], tcap[r]) : Lk[r * kLS + kq - 1];
-      if (r >= mq) thr = -kInf;
-      else if (tk == kInf) thr = kMaxF;
-      else if (METRIC == KNN_METRIC_EUCLIDEAN) {
-        const float myn = qn[r];
-        thr = fminf((tk - myn) + kSlack * (fabsf(tk) + myn + cm), kMaxF);
-      } else {
-        thr = fminf((tk - 1.f) + kSlack * (fabsf(tk) + 2.f), kMaxF);
+  if (warp < 4 * QT) {
+    // ------------------------------------------------ epilogue: a thread per row
+    const int qt = warp >> 2, quarter = warp & 3;
+    const uint32_t tlane = (uint32_t)(quarter * 32) << 16;
+    const int row = q0 + qt * kBM + quarter * 32 + lane;  // row of the leaf
+    const bool live = row < nq;
+    const int64_t pos = lo + row;  // position in the tree's order
+    const int qid = live ? a.perm[pos] : -1;
+    const float myn = METRIC == KNN_METRIC_EUCLIDEAN && live ? a.np[pos] : 0.f;
+    if (!stopped && qt < qts) {
+      // the row's 16-bit elements into tensor memory, two per 32-bit column
+      const uint16_t* src = a.Xp + (size_t)(live ? pos : lo) * a.ldr;
+#pragma unroll
+      for (int ch = 0; ch < NCH; ++ch) {
+        uint32_t v[32];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          uint4 q = make_uint4(0u, 0u, 0u, 0u);
+          const int e = ch * kKC + 8 * u;
+          if (live && e < a.ldr) q = __ldg(reinterpret_cast<const uint4*>(src + e));
+          v[4 * u] = q.x;
+          v[4 * u + 1] = q.y;
+          v[4 * u + 2] = q.z;
+          v[4 * u + 3] = q.w;
+        }
+        tmem_st32(tmem + tlane + (uint32_t)(Plan::kA0 + qt * Plan::kA + ch * 32), v);
       }
-    }
-#pragma unroll 1
-    for (int ri = 0; ri < 2; ++ri) {
-      const int col0 = ri * kRound + half * 32;  // this thread's 32 columns
-      if (ri * kRound >= mc) {                   // warp-uniform: no candidates in this round
-        if (pass == 1) msk[r * 4 + ri * 2 + half] = 0u;
-        continue;
-      }
-      uint32_t v[32];
-      tmem_ld32(tq + (uint32_t)col0, v);
-      const float4* cn4 = reinterpret_cast<const float4*>(cn + col0);
-      if (FIRST && pass == 0) {
-        // smallest exact key of these 32 columns (the row's own column
-        // left out) into the slice's group
-        const float myn = qn[r];
-        const int64_t sb = (lo + q0 + r) - blo - c0 - col0;
-        float m = kInf;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 c = cn4[q];
-          const float cc[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float dot = __uint_as_float(v[4 * q + e]);
-            const float key = METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(myn, cc[e]))
-                                                             : __fsub_rn(1.f + cc[e], dot);
-            m = (sb == 4 * q + e) ? m : fminf(m, key);
-          }
-        }
-        const int g = ((c0 / kBN) * 4 + ri * 2 + half) & (kGroups - 1);
-        gm[r * kGS + g] = fminf(gm[r * kGS + g], m);
-      } else {
-        // bit j of neg = sign of thr - key'_j, shifted in from column 31 down
-        uint32_t neg = 0;
-#pragma unroll
-        for (int q = 7; q >= 0; --q) {
-          const float4 c = cn4[q];
-          const float cc[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-          for (int e = 3; e >= 0; --e) {
-            const float dot = __uint_as_float(v[4 * q + e]);
-            const float kp =
-                METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, cc[e]) : __fsub_rn(cc[e], dot);
-            neg = __funnelshift_l(__float_as_uint(__fsub_rn(thr, kp)), neg, 1);
-          }
-        }
-        uint32_t mask = ~neg;
-        // the row's own point (its leaf lies inside the block) never survives
-        const int64_t selfbit = (lo + q0 + r) - blo - c0 - col0;
-        if (selfbit >= 0 && selfbit < 32) mask &= ~(1u << (int)selfbit);
-        if (glog) {  // grouped leaves: the row's own leaf's columns only
-          const int a = min(max((int)rcol[2 * r] - (c0 + col0), 0), 32);
-          const int b = min(max((int)rcol[2 * r + 1] - (c0 + col0), 0), 32);
-          mask &= (uint32_t)(((1ull << b) - 1ull) ^ ((1ull << a) - 1ull));
-        }
-        if (xcl) {
-          // listed ids among these 32 columns: walk the row's sorted
-          // positions (each thread's columns only increase)
-          const int lo_c = c0 + col0;
-          uint32_t ex = 0;
-          int p = xp[r * kXS + xptr];
-          while (p < lo_c + 32) {
-            if (p >= lo_c) ex |= 1u << (p - lo_c);
-            p = xp[r * kXS + (++xptr)];
-          }
-          mask &= ~ex;
-        }
-        msk[r * 4 + ri * 2 + half] = mask;
-      }
-    }
-    // step s + 1's operand (staged since [A]) lands before [B]; its MMA is
-    // issued after [B] and runs while this step's survivors are merged
-    if (has_next) {
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();  // [B]
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (has_next && tid == 0) issue_mma(s + 1);
-    if (pass == 1) {
-      // The quarter's rows with survivors (one ballot) alternate between
-      // its two warps; survivors' products come from the warp's lane
-      // quarter of tensor memory.
-      const int rowq = quarter * 32 + lane;
-      const bool has = rowq < mq && (msk[rowq * 4] | msk[rowq * 4 + 1] | msk[rowq * 4 + 2] | msk[rowq * 4 + 3]) != 0;
-      const uint32_t all = __ballot_sync(0xFFFFFFFFu, has);
-      const bool mine = has && (__popc(all & ((1u << lane) - 1u)) & 1) == half;
-      uint32_t rows = __ballot_sync(0xFFFFFFFFu, mine);
-      while (rows) {
-        const int ql = __ffs(rows) - 1;  // row within the quarter
-        const int qq = quarter * 32 + ql;
-        rows &= rows - 1;
-        float lk = Lk[qq * kLS + lane];
-        uint32_t li = Li[qq * kLS + lane];
-        const float myn = qn[qq];
+    __syncthreads();  // queries in place: MMAs may start
+    if (!stopped && qt < qts) {
+      const float kInf = __int_as_float(0x7F800000);
+      const float kMaxF = __int_as_float(0x7F7FFFFF);
+      unsigned char* mine = warp_area + (size_t)warp * kWarpBytes;
+      unsigned char* dump = mine + lane * kDumpStride;                 // this row's slice
+      uint32_t* bits = reinterpret_cast<uint32_t*>(mine + kWarpDump);  // [32][kBandWords]
+      float* gm = reinterpret_cast<float*>(mine);                      // [32][kGS] during pass 0
+      const size_t slot = (size_t)blockIdx.x * (kBM * QT) + warp * 32;  // the warp's rows in the scratch
+      uint2* surv = a.surv + slot * kCap;
+      uint2* mysurv = surv + lane * kCap;
+      const int self = (int)(pos - blo);  // the row's own column (its leaf lies inside the block)
+      int ca = 0, cb = nb;                // grouped leaves: the row's own leaf's columns
+      if (a.glog) {
+        int64_t s = lo, e = range.hi;
+        for (int g = 0; g < (1 << a.glog); ++g) {
+          const int64_t end = range.seg.off + node_lo(range.seg.n, range.seg.depth, range.j + g + 1);
+          if (pos < end) {
+            e = end;
+            break;
+          }
+          s = end;
+        }
+        ca = (int)(s - blo);
+        cb = (int)(e - blo);
+      }
+      float tk = kInf;          // bound on the row's kq-th key: its list tail, or the bounding pass's
+      float cm_all = 0.f;       // largest |y|^2 met in the bounding pass
+      int cnt = 0;              // buffered survivors
+      uint32_t have = FIRST ? 0u : 0xFFFFFFFFu;  // rows whose list holds something
+      // later trees: the bitmap, for every row, of the columns in [band, band + kBand)
+      // that hold an id of the row's list
+      const int wrows = min(32, nq - (row - lane));  // rows of this warp (<= 0: none)
+      auto set_band = [&](int band) {
+        int32_t p[32];
+        const int32_t* src = a.plist + (size_t)(pos - lane) * a.kq + lane;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) p[i] = i < wrows && lane < a.kq ? __ldg(src + (size_t)i * a.kq) : -1;
+        __syncwarp();
+        for (int e = lane; e < 32 * kBandWords; e += 32) bits[e] = 0u;
+        __syncwarp();
+        const int32_t base = (int32_t)(blo + band);  // positions fit 31 bits
+        const uint32_t width = (uint32_t)min(kBand, nb - band);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const uint32_t c = (uint32_t)(p[i] - base);  // -1 and columns before the band wrap past width
+          if (p[i] >= 0 && c < width) atomicOr(&bits[i * kBandWords + (c >> 5)], 1u << (c & 31));
+        }
+        __syncwarp();
+      };
+      if (!FIRST) {
+        if (live) tk = from_orderable(a.akey[(size_t)qid * a.kq + a.kq - 1]);
+        if (!(tk < kInf)) tk = kInf;  // free slots
+      }
+      if (npre) {
+#pragma unroll 8
+        for (int e = 0; e < kGroups; ++e) gm[lane * kGS + e] = kInf;
+      }
+      bool ok = true;
 #pragma unroll 1
-        for (int h = 0; h < 4; ++h) {
-          uint32_t bal = msk[qq * 4 + h];
-          if (bal == 0) continue;
-          const int cb = h * 32;  // the slice's first column in the tile
-          if (FIRST && __popc(bal) >= kBulkMerge) {
-            // lane j <- product of column cb + j of row qq
-            uint32_t v[32];
-            tmem_ld32(tq + (uint32_t)cb, v);
-            float dot = 0.f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float t = __shfl_sync(0xFFFFFFFFu, __uint_as_float(v[j]), ql);
-              if (lane == j) dot = t;
-            }
-            float ck = kInf;
-            uint32_t ci = kNoId;
-            if ((bal >> lane) & 1u) {
-              ck = METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(myn, cn[cb + lane]))
-                                                  : __fsub_rn(1.f, dot);
-              ci = (uint32_t)cid[cb + lane];
-            }
-            warp_bitonic_sort32(ck, ci);
-            warp_merge_lower(lk, li, ck, ci);
-            continue;
-          }
-          while (bal) {
-            const int j = __ffs(bal) - 1;
-            bal &= bal - 1;
-            const float dot = __shfl_sync(0xFFFFFFFFu, __uint_as_float(tmem_ld1(tq + (uint32_t)(cb + j))), ql);
-            const float k1 = METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(myn, cn[cb + j]))
-                                                            : __fsub_rn(1.f, dot);
-            const uint32_t i1 = (uint32_t)cid[cb + j];
-            const bool dup = !FIRST && !xcl && __ballot_sync(0xFFFFFFFFu, lane < kq && li == i1) != 0;
-            if (!dup) warp_insert1(lk, li, k1, i1);
-          }
+      for (int s = 0; s < nsteps; ++s) {
+        const bool pre = PRE && s < npre;
+        const int t = s < npre ? s : s - npre;
+        const int buf = s % NB;
+        const uint32_t acc = (uint32_t)(qt * NB + buf);
+        if (!FIRST && !pre && t * kTN % kBand == 0) set_band(t * kTN);
+        if (METRIC == KNN_METRIC_EUCLIDEAN)
+          ok = mbar_wait(bar_nfull + 8 * (s % kNormSlots), (uint32_t)(s / kNormSlots) & 1u, status, a.err);
+        ok = ok && mbar_wait(bar_afull + 8 * acc, (uint32_t)(s / NB) & 1u, status, a.err);
+        ok = __all_sync(0xFFFFFFFFu, ok);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const float* tn = tnorms + (s % kNormSlots) * (kTN + 4);
+        const float cm = METRIC == KNN_METRIC_EUCLIDEAN ? tn[kTN] : 0.f;
+        float thr = kMaxF;  // the row's filter bound
+        if (tk < kInf) {
+          if (METRIC == KNN_METRIC_EUCLIDEAN) thr = fminf((tk - myn) + kSlack * (fabsf(tk) + myn + cm), kMaxF);
+          else thr = fminf((tk - 1.f) + kSlack * (fabsf(tk) + 2.f), kMaxF);
         }
-        Lk[qq * kLS + lane] = lk;
-        Li[qq * kLS + lane] = li;
+        const uint64_t thr2 = pack2(__float_as_uint(thr), __float_as_uint(thr));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c0 = t * kTN + h * 32;  // the slice's first column
+          uint32_t v[32];
+          tmem_ld32(tmem + tlane + acc * kTN + (uint32_t)(h * 32), v);
+          tmem_wait_ld(v);
+          if (h == 1) {  // the accumulator is free
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_aempty + 8 * acc);
+          }
+          const ulonglong2* n4 = reinterpret_cast<const ulonglong2*>(tn + h * 32);  // four columns each
+          // last use of the tile's norms by this warp (after the reads below)
+          auto norms_done = [&]() {
+            if (METRIC == KNN_METRIC_EUCLIDEAN && h == 1) {
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar_nempty + 8 * (s % kNormSlots));
+            }
+          };
+          const int own = self - c0;
+          const int lim = nb - c0;  // columns of the block from c0 on
+          if (pre) {
+            // smallest key' of the slice, the row's own column and the columns
+            // past the block left out, into the slice's group
+            cm_all = fmaxf(cm_all, cm);
+            float m = kInf;
+            if (__any_sync(0xFFFFFFFFu, own >= 0 && own < 32) || lim < 32) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) {
+                const float kp = METRIC == KNN_METRIC_EUCLIDEAN
+                                     ? -__fmaf_rn(2.f, __uint_as_float(v[c]), tn[h * 32 + c])
+                                     : -__uint_as_float(v[c]);
+                m = c == own || c >= lim ? m : fminf(m, kp);
+              }
+            } else {
+              float big[4] = {-kInf, -kInf, -kInf, -kInf};
+#pragma unroll
+              for (int c = 0; c < 32; c += 4) {
+                uint32_t d[4] = {v[c], v[c + 1], v[c + 2], v[c + 3]};
+                if (METRIC == KNN_METRIC_EUCLIDEAN) {
+                  const ulonglong2 n = n4[c >> 2];
+                  unpack2(fma2(pack2(0x40000000u, 0x40000000u), pack2(d[0], d[1]), n.x), d[0], d[1]);
+                  unpack2(fma2(pack2(0x40000000u, 0x40000000u), pack2(d[2], d[3]), n.y), d[2], d[3]);
+                }
+                float& b0 = big[(c >> 1) & 3];
+                float& b1 = big[((c >> 1) & 3) + 1];
+                b0 = fmaxf(b0, fmaxf(__uint_as_float(d[0]), __uint_as_float(d[1])));
+                b1 = fmaxf(b1, fmaxf(__uint_as_float(d[2]), __uint_as_float(d[3])));
+              }
+              m = -fmaxf(fmaxf(big[0], big[1]), fmaxf(big[2], big[3]));
+            }
+            norms_done();
+            float* group = gm + lane * kGS + ((2 * s + h) & (kGroups - 1));
+            *group = fminf(*group, m);
+            if (h == 1 && s == npre - 1) {
+              // bound per row: the kq-th smallest of its group minima (kBoundRows
+              // rows interleaved).  Each row's 64 minima: lanes' first halves sorted
+              // ascending, second halves descending, their lane-wise minima are
+              // the 32 smallest (a bitonic sequence), merged.
+              __syncwarp();
+              float bound = kInf;
+#pragma unroll 1
+              for (int i0 = 0; i0 < 32; i0 += kBoundRows) {
+                float x[kBoundRows], y[kBoundRows];
+#pragma unroll
+                for (int i = 0; i < kBoundRows; ++i) {
+                  x[i] = gm[(i0 + i) * kGS + lane];
+                  y[i] = gm[(i0 + i) * kGS + 32 + lane];
+                }
+#pragma unroll 1
+                for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll 1
+                  for (int m = size >> 1; m >= 1; m >>= 1) {
+                    const bool keep_min = ((lane & size) == 0) == ((lane & m) == 0);
+#pragma unroll
+                    for (int i = 0; i < kBoundRows; ++i) {
+                      const float ox = __shfl_xor_sync(0xFFFFFFFFu, x[i], m);
+                      const float oy = __shfl_xor_sync(0xFFFFFFFFu, y[i], m);
+                      x[i] = keep_min ? fminf(x[i], ox) : fmaxf(x[i], ox);
+                      y[i] = keep_min ? fmaxf(y[i], oy) : fminf(y[i], oy);
+                    }
+                  }
+                }
+#pragma unroll
+                for (int i = 0; i < kBoundRows; ++i) x[i] = fminf(x[i], y[i]);
+#pragma unroll 1
+                for (int m = 16; m >= 1; m >>= 1) {
+                  const bool keep_min = (lane & m) == 0;
+#pragma unroll
+                  for (int i = 0; i < kBoundRows; ++i) {
+                    const float o = __shfl_xor_sync(0xFFFFFFFFu, x[i], m);
+                    x[i] = keep_min ? fminf(x[i], o) : fmaxf(x[i], o);
+                  }
+                }
+#pragma unroll
+                for (int i = 0; i < kBoundRows; ++i) {
+                  const float b = __shfl_sync(0xFFFFFFFFu, x[i], a.kq - 1);
+                  if (lane == i0 + i) bound = b;
+                }
+              }
+              // key' -> key units, widened past the rounding of both
+              const float cap = METRIC == KNN_METRIC_EUCLIDEAN
+                                    ? (bound + myn) + kSlack * (fabsf(bound) + 2.f * myn + cm_all)
+                                    : (bound + 1.f) + kSlack * (fabsf(bound) + 2.f);
+              if (cap < tk) tk = cap;
+              __syncwarp();
+            }
+          } else {
+            // bit c of neg = sign of thr - key'_c, shifted in from the highest column
+            // down, in four independent chains of eight columns
+            uint32_t part[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int c = 4; c >= 0; c -= 4)
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const int e = 8 * q + c;
+                // -key' = 2 x.y - |y|^2 (EUCLIDEAN) or x.y (COSINE)
+                uint64_t lo2 = pack2(v[e], v[e + 1]), hi2 = pack2(v[e + 2], v[e + 3]);
+                if (METRIC == KNN_METRIC_EUCLIDEAN) {
+                  const ulonglong2 n = n4[e >> 2];
+                  lo2 = fma2(pack2(0x40000000u, 0x40000000u), lo2, n.x);
+                  hi2 = fma2(pack2(0x40000000u, 0x40000000u), hi2, n.y);
+                }
+                uint32_t s0, s1, s2, s3;
+                unpack2(add2(thr2, lo2), s0, s1);
+                unpack2(add2(thr2, hi2), s2, s3);
+                part[q] = __funnelshift_l(s3, part[q], 1);
+                part[q] = __funnelshift_l(s2, part[q], 1);
+                part[q] = __funnelshift_l(s1, part[q], 1);
+                part[q] = __funnelshift_l(s0, part[q], 1);
+              }
+            const uint32_t neg = part[0] | (part[1] << 8) | (part[2] << 16) | (part[3] << 24);
+            norms_done();
+            uint32_t m = live ? ~neg : 0u;
+            if (own >= 0 && own < 32) m &= ~(1u << own);
+            if (lim < 32) m &= lim <= 0 ? 0u : (1u << lim) - 1u;
+            if (a.glog) {  // grouped leaves: the row's own leaf's columns only
+              const int lo_c = min(max(ca - c0, 0), 32), hi_c = min(max(cb - c0, 0), 32);
+              m &= (uint32_t)(((1ull << hi_c) - 1ull) ^ ((1ull << lo_c) - 1ull));
+        }
+            if (!FIRST) m &= ~bits[lane * kBandWords + (c0 % kBand) / 32];
+            const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, m);
+            if (any) {
+              // the products through shared memory (a lane cannot index its registers);
+              // then every lane appends its own survivors
+#pragma unroll
+              for (int c = 0; c < 32; c += 4)
+                *reinterpret_cast<uint4*>(dump + 4 * c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+              for (uint32_t left = m; left; left &= left - 1) {
+                const int c = __ffs(left) - 1;
+                mysurv[cnt++] = make_uint2(*reinterpret_cast<const uint32_t*>(dump + 4 * c), (uint32_t)(c0 + c));
+              }
+        }
+        }
+        }
+        // a buffer too full for another tile is merged here (rare), with the
+        // other well filled ones
+        if (pre || !__any_sync(0xFFFFFFFFu, cnt > kFlushAt)) continue;
+        const uint32_t rows = __ballot_sync(0xFFFFFFFFu, cnt >= kFlushMin);
+        tk = merge_survivors<METRIC>(a.akey, a.aid, a.np + blo, a.perm + blo, a.kq, surv, qid, myn, cnt, tk, have, rows);
+        have |= rows;
+        if ((rows >> lane) & 1u) cnt = 0;
       }
+      if (ok) a.count[slot + lane] = (uint32_t)cnt | (FIRST && ((have >> lane) & 1u) ? kListed : 0u);
     }
+  } else {
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    if (FIRST && pass == 0 && s == ntiles - 1) {
-      // bound per row: the kq-th smallest of its group minima (warp w: rows
-      // w + 8 i, four rows' networks interleaved).  Each row's 64 minima:
-      // lanes' first halves sorted ascending, second halves descending, their
-      // lane-wise minima are the 32 smallest (a bitonic sequence), merged.
-      // Then the lists start empty for pass 1.
-      for (int i0 = 0; i0 < kBM / 8; i0 += 4) {
-        float a[4], b[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int qq = warp + 8 * (i0 + i);
-          a[i] = gm[qq * kGS + lane];
-          b[i] = gm[qq * kGS + 32 + lane];
+    __syncthreads();  // queries in place
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    // Whole warps run these loops and one elected lane issues: the operands of
+    // the TMA and MMA instructions stay in uniform registers.
+    if (!stopped && warp == 4 * QT) {
+      // ----------------------------------------------------------- producer
+      const uint32_t ring0 = __shfl_sync(0xFFFFFFFFu, smem_u32(ring), 0);
+      uint32_t q = 0;
+      bool ok = true;
+      // -|y|^2 of a tile's columns (EUCLIDEAN), -inf past the block, fetched a tile ahead
+      const float kInf = __int_as_float(0x7F800000);
+      float f0 = 0.f, f1 = 0.f;
+      auto fetch_norms = [&](int s) {
+        const int c = (s < npre ? s : s - npre) * kTN + lane;
+        f0 = c < nb ? a.np[blo + c] : kInf;
+        f1 = c + 32 < nb ? a.np[blo + c + 32] : kInf;
+      };
+      if (METRIC == KNN_METRIC_EUCLIDEAN) fetch_norms(0);
+      for (int s = 0; ok && s < nsteps; ++s) {
+        const int t = s < npre ? s : s - npre;
+        if (METRIC == KNN_METRIC_EUCLIDEAN) {
+          const int slot = s % kNormSlots, round = s / kNormSlots;
+          if (round > 0) ok = mbar_wait(bar_nempty + 8 * slot, (uint32_t)(round - 1) & 1u, status, a.err);
+          if (!__all_sync(0xFFFFFFFFu, ok)) {
+            ok = false;
+            break;
+          }
+          float* tn = tnorms + slot * (kTN + 4);
+          tn[lane] = -f0;
+          tn[lane + 32] = -f1;
+          // norms are >= 0, so their bit patterns order as unsigned integers
+          const float fm = fmaxf(f0 < kInf ? f0 : 0.f, f1 < kInf ? f1 : 0.f);
+          const uint32_t big = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(fm));
+          if (lane == 0) tn[kTN] = __uint_as_float(big);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_nfull + 8 * slot);
+          if (s + 1 < nsteps) fetch_norms(s + 1);
         }
+        for (int ch = 0; ch < NCH; ++ch, ++q) {
+          const uint32_t st = q % RING, round = q / RING;
+          if (round > 0) ok = mbar_wait(bar_empty + 8 * st, (round - 1) & 1u, status, a.err);
+          if (!__all_sync(0xFFFFFFFFu, ok)) {
+            ok = false;
+            break;
+          }
+          if (elect_one()) {
+            mbar_expect_tx(bar_full + 8 * st, kBoxBytes);
+            tma_load_box(ring0 + st * kBoxBytes, &bmap, ch * kKC, (int)(blo + (int64_t)t * kTN), bar_full + 8 * st);
+          }
+          __syncwarp();
+        }
+      }
+      // the block's last loads land before it may end
+      for (uint32_t d = q < (uint32_t)RING ? 0u : q - RING; d < q; ++d) {
+        const uint64_t t0 = global_ns();
+        while (!mbar_try_wait(bar_full + 8 * (d % RING), (d / RING) & 1u) && global_ns() - t0 < kWaitNs) {
+        }
+      }
+    } else if (!stopped) {
+      // ---------------------------------------------------------------- MMA
+      const uint32_t ring0 = __shfl_sync(0xFFFFFFFFu, smem_u32(ring), 0);
+      const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
+      uint32_t q = 0;
+      bool ok = true;
+      for (int s = 0; ok && s < nsteps; ++s) {
+        // one query tile after the other: the next one's products need not wait for
+        // this one's accumulator
+        const int buf = s % NB, use = s / NB;
+        for (int qt = 0; ok && qt < qts; ++qt) {
+          if (use > 0) ok = mbar_wait(bar_aempty + 8 * (qt * NB + buf), (uint32_t)(use - 1) & 1u, status, a.err);
+          const uint32_t d = tm + (uint32_t)((qt * NB + buf) * kTN);
+          const uint32_t qa = tm + (uint32_t)(Plan::kA0 + qt * Plan::kA);
 #pragma unroll
-        for (int size = 2; size <= 32; size <<= 1) {
+          for (int ch = 0; ch < NCH; ++ch) {
+            const uint32_t st = (q + ch) % RING;
+            if (qt == 0) ok = ok && mbar_wait(bar_full + 8 * st, ((q + ch) / RING) & 1u, status, a.err);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const int steps = min(kKC / 16, a.ksteps - ch * (kKC / 16));
+            const uint64_t b0 = desc_sw128(ring0 + st * kBoxBytes);
+            if (elect_one()) {
 #pragma unroll
-          for (int m = size >> 1; m >= 1; m >>= 1) {
-            const bool keep_min = ((lane & size) == 0) == ((lane & m) == 0);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float oa = __shfl_xor_sync(0xFFFFFFFFu, a[i], m);
-              const float ob = __shfl_xor_sync(0xFFFFFFFFu, b[i], m);
-              a[i] = keep_min ? fminf(a[i], oa) : fmaxf(a[i], oa);
-              b[i] = keep_min ? fmaxf(b[i], ob) : fminf(b[i], ob);
+              for (int kk = 0; kk < kKC / 16; ++kk)
+                if (kk < steps)
+                  umma_f16_ts(d, qa + ch * 32 + kk * 8, b0 + (uint64_t)(kk * 2), a.idesc, (ch | kk) != 0 ? 1u : 0u);
+              if (qt == qts - 1) umma_commit(bar_empty + 8 * st);
+              if (ch == NCH - 1) umma_commit(bar_afull + 8 * (qt * NB + buf));
             }
+            __syncwarp();
           }
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = fminf(a[i], b[i]);
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1) {
-          const bool keep_min = (lane & m) == 0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float o = __shfl_xor_sync(0xFFFFFFFFu, a[i], m);
-            a[i] = keep_min ? fminf(a[i], o) : fmaxf(a[i], o);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float t = __shfl_sync(0xFFFFFFFFu, a[i], kq - 1);
-          if (lane == 0) tcap[warp + 8 * (i0 + i)] = t;
-        }
+        q += NCH;
       }
-      __syncthreads();
-      for (int e = tid; e < kBM * kLS; e += kUThreads) {
-        Lk[e] = kInf;
-        Li[e] = kNoId;
+      // every issued product completes before tensor memory is freed
+      if (elect_one()) umma_commit(bar_done);
+      __syncwarp();
+      const uint64_t t0 = global_ns();
+      while (!mbar_try_wait(bar_done, 0) && global_ns() - t0 < kWaitNs) {
       }
     }
-  }
-  // the last step's merge is ordered before the write-back only by this barrier
-  __syncthreads();
-  if (*status == 0) {
-    for (int e = tid; e < kBM * 32; e += kUThreads) {
-      const int r = e >> 5, s = e & 31;
-      const int32_t id = qid[r];
-      if (id >= 0 && s < kq) {
-        akey[(size_t)id * kq + s] = Lk[r * kLS + s];
-        aid[(size_t)id * kq + s] = Li[r * kLS + s];
-      }
-    }
+    __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
-    __syncwarp();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(*tmem_slot), "r"(kTmemCols));
+  if (warp == 4 * QT + 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)Plan::kTotal));
   }
+}
+
+// The survivors that k_leaf_tc left, into the lists: a warp takes 32 rows, the
+// rows with survivors (first tree: every row) kMergeRows at a time.  A kernel
+// of its own, so that sorting and merging run at full occupancy instead of in
+// the few warps that share an SM with the tiles, and never stall the products.
+template <int METRIC, bool FIRST, int QT>
+__global__ void __launch_bounds__(kBM * QT) k_leaf_tc_merge(const __grid_constant__ LeafTcArgs a) {
+  const BlockRange range = block_range<QT>(a, a.block0 + blockIdx.x);
+  const int lane = threadIdx.x & 31;
+  const int row = range.q0 + (int)threadIdx.x;
+  const bool live = row < (int)(range.hi - range.lo);
+  if (*reinterpret_cast<volatile int*>(a.err) != 0) return;  // the build gave up: counts may be missing
+  const size_t slot = (size_t)blockIdx.x * (kBM * QT) + threadIdx.x;
+  uint32_t c = live ? a.count[slot] : 0u;
+  const uint32_t rows = __ballot_sync(0xFFFFFFFFu, live && (FIRST ? c != kListed : c != 0u));
+  if (rows == 0) return;
+  const uint32_t have = FIRST ? __ballot_sync(0xFFFFFFFFu, (c & kListed) != 0u) : 0xFFFFFFFFu;
+  const int64_t pos = range.lo + row;
+  const int qid = live ? a.perm[pos] : -1;
+  const float myn = METRIC == KNN_METRIC_EUCLIDEAN && live ? a.np[pos] : 0.f;
+  merge_survivors<METRIC>(a.akey, a.aid, a.np + range.blo, a.perm + range.blo, a.kq, a.surv + (slot - lane) * kCap,
+                          qid, myn, (int)(c & ~kListed), 0.f, have, rows);
 }
 
 // inv[order[i]] = i: the position of each point in a tree's order.
@@ -723,13 +997,13 @@ __device__ __forceinline__ float from_operand(uint16_t b, bool f16) {
   return f16 ? __half2float(__ushort_as_half(b)) : __bfloat162float(__ushort_as_bfloat16(b));
 }
 
-// 16-bit operand copy: rows of Kp BF16 or FP16 values (zero padded), COSINE
+// 16-bit operand copy: rows of ldr BF16 or FP16 values (zero padded), COSINE
 // rows divided by their FP32 norm first; norms2 = |row|^2 of the rounded
 // values (EUCLIDEAN).  FP16 EUCLIDEAN rows are first multiplied by the power
 // of two 2^e that brings the largest |x| (maxabs) into [2^14, 2^15), inside
 // the FP16 range: a power-of-two scale is exact, scales every key of the tile
 // stage by the same 2^2e and so keeps its ranking (the re-rank uses X).
-__global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int dpad, int Kp, int metric, bool f16,
+__global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int dpad, int ldr, int metric, bool f16,
                              const unsigned int* __restrict__ maxabs, const float* __restrict__ norms,
                              uint16_t* __restrict__ Xb, float* __restrict__ norms2) {
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -750,16 +1024,44 @@ __global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int 
     scale = ldexpf(1.f, e);
   }
   float s = 0.f;
-  for (int c = lane; c < Kp; c += 32) {
+  for (int c = lane; c < ldr; c += 32) {
     const float v = c < d ? X[(size_t)row * dpad + c] : 0.f;
     const uint16_t b = to_operand(__fmul_rn(v, scale), f16);
-    Xb[(size_t)row * Kp + c] = b;
+    Xb[(size_t)row * ldr + c] = b;
     const float f = from_operand(b, f16);
     s = __fmaf_rn(f, f, s);
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, off));
   if (lane == 0) norms2[row] = s;
+}
+
+// A tree's order: Xp[i] = Xb[perm[i]], np[i] = norms2[perm[i]]; one thread per
+// 16-byte unit (units per row: ldr / 8).
+__global__ void __launch_bounds__(256) k_permute_operand(const uint4* __restrict__ Xb,
+                                                         const float* __restrict__ norms2,
+                                                         const int32_t* __restrict__ perm, int64_t n, int units,
+                                                         uint4* __restrict__ Xp, float* __restrict__ np) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n * units) return;
+  const int64_t i = g / units;
+  const int u = (int)(g - i * units);
+  const int32_t id = __ldg(perm + i);
+  Xp[g] = __ldg(Xb + (size_t)id * units + u);
+  if (u == 0) np[i] = norms2[id];
+}
+
+// Positions in a tree's order of every entry of every point's list, rows in
+// that order too (-1: empty): plist[p][e] = inv[aid[perm[p]][e]].
+__global__ void __launch_bounds__(256) k_list_positions(const uint32_t* __restrict__ aid,
+                                                        const int32_t* __restrict__ perm,
+                                                        const int32_t* __restrict__ inv, int64_t n, int kq,
+                                                        int32_t* __restrict__ plist) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n * kq) return;
+  const int64_t p = g / kq;
+  const uint32_t id = aid[(size_t)__ldg(perm + p) * kq + (int)(g - p * kq)];
+  plist[g] = id < (uint64_t)n ? __ldg(inv + id) : -1;
 }
 
 // Exact FP32 keys (the reference's order) of each point's kq approximate
@@ -781,7 +1083,9 @@ __global__ void __launch_bounds__(256) k_rerank(const float* __restrict__ X, int
   const float kInf = __int_as_float(0x7F800000);
   const float4* xr = reinterpret_cast<const float4*>(X + (size_t)i * dpad);
   for (int c = lane; c < (dpad >> 2); c += 32) reinterpret_cast<float4*>(xq)[c] = xr[c];
-  const uint32_t cj = lane < kq ? aid[(size_t)i * kq + lane] : kNoId;
+  // an id outside [0, n) is an empty entry
+  uint32_t cj = lane < kq ? aid[(size_t)i * kq + lane] : kNoId;
+  if (cj >= (uint64_t)n) cj = kNoId;
   const bool valid = cj != kNoId;
   ids[lane] = cj;
   __syncwarp();
@@ -826,16 +1130,102 @@ __global__ void __launch_bounds__(256) k_rerank(const float* __restrict__ X, int
   }
 }
 
-size_t umma_smem_bytes(int Kp) {
-  // alignment slack + A + B + lists + (qid, qn) + two steps' (cid, cn) + survivor masks + two
-  // steps' norm maxima + listed columns + first-tree bounds + barrier words
-  return 1024 + 2 * (size_t)(Kp / kKC) * kChunkBytes + (size_t)kBM * kLS * 8 + (size_t)kBM * 8 +
-         (size_t)kBN * 3 * 8 + (size_t)kBM * 4 * 4 + 48 + (size_t)kBM * kXS * 2 + (size_t)kBM * 4 + 64;
+namespace {
+
+template <int NCH, int QT>
+size_t leaf_tc_smem() {
+  return 1024 + (size_t)kRing * kBoxBytes + (size_t)4 * QT * kWarpBytes + kNormBytes +
+         8 * (2 * kRing + 2 * QT * TmemPlan<NCH, QT>::kNB + 2 * kNormSlots + 1) + 16;
 }
 
+// 2-D map of the 16-bit rows [n][ldr]: boxes of 64 rows x 64 elements, zeros
+// outside (past the last row and past column ldr).
+bool operand_map(const void* Xp, int64_t n, int ldr, bool f16, CUtensorMap* map) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static Encode encode = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<Encode>(f);
+  }();
+  if (!encode) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)ldr, (cuuint64_t)n};
+  const cuuint64_t strides[1] = {(cuuint64_t)ldr * 2};
+  const cuuint32_t box[2] = {kKC, kTN};
+  const cuuint32_t one[2] = {1, 1};
+  return encode(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                const_cast<void*>(Xp), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// A tree's tiles, kChunkRows rows at a time, each chunk followed by its merge.
+template <int METRIC, bool FIRST, bool PRE, int NCH, int QT>
+void launch_tc(const CUtensorMap& map, LeafTcArgs t, int64_t blocks, cudaStream_t st, LaunchLog& log) {
+  const size_t smem = leaf_tc_smem<NCH, QT>();
+  cudaFuncSetAttribute(k_leaf_tc<METRIC, FIRST, PRE, NCH, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int64_t chunk = kChunkRows / (kBM * QT);
+  for (t.block0 = 0; t.block0 < blocks; t.block0 += chunk) {
+    const unsigned grid = (unsigned)std::min(chunk, blocks - t.block0);
+    k_leaf_tc<METRIC, FIRST, PRE, NCH, QT><<<grid, 64 + 128 * QT, smem, st>>>(map, t);
+    k_leaf_tc_merge<METRIC, FIRST, QT><<<grid, kBM * QT, 0, st>>>(t);
+    log.add(2);
+  }
+}
+template <int METRIC, bool FIRST, bool PRE>
+void launch_tc_tiles(int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks, cudaStream_t st,
+                     LaunchLog& log) {
+  if (qt == 2 && nch == 1) launch_tc<METRIC, FIRST, PRE, 1, 2>(map, t, blocks, st, log);
+  else if (qt == 2) launch_tc<METRIC, FIRST, PRE, 2, 2>(map, t, blocks, st, log);
+  else if (nch == 1) launch_tc<METRIC, FIRST, PRE, 1, 1>(map, t, blocks, st, log);
+  else if (nch == 2) launch_tc<METRIC, FIRST, PRE, 2, 1>(map, t, blocks, st, log);
+  else if (nch == 3) launch_tc<METRIC, FIRST, PRE, 3, 1>(map, t, blocks, st, log);
+  else launch_tc<METRIC, FIRST, PRE, 4, 1>(map, t, blocks, st, log);
+}
+template <int METRIC>
+void launch_tc_tree(int tree, bool pre, int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks,
+                    cudaStream_t st, LaunchLog& log) {
+  if (tree == 0) launch_tc_tiles<METRIC, true, true>(qt, nch, map, t, blocks, st, log);
+  else if (pre) launch_tc_tiles<METRIC, false, true>(qt, nch, map, t, blocks, st, log);
+  else launch_tc_tiles<METRIC, false, false>(qt, nch, map, t, blocks, st, log);
+}
+
+}  // namespace
+
+namespace {
+// Query tiles per block and blocks per leaf (or per group of sibling leaves).
+// Two query tiles share every candidate box, which halves the L2 reads (integer
+// mixture, 8 trees, leaf 2048, tiles without the second bounding pass: 14.9 ms
+// against 15.1 with one; 10M x 96 COSINE 194 against 199); one where leaves (or
+// groups of them) fill a single tile, and above 128 dims, where two query tiles
+// would take all of tensor memory.
+struct TcShape {
+  int qt, qtiles, glog;
+};
+TcShape tc_shape(const UmmaLeafArgs& a) {
+  TcShape s;
+  s.glog = a.tc_group >= 4 ? 2 : a.tc_group == 2 ? 1 : 0;
+  s.qt = a.d > 2 * kKC || s.glog || a.maxleaf <= kBM ? 1 : 2;
+  s.qtiles = s.glog ? 1 : (int)((a.maxleaf + kBM * s.qt - 1) / (kBM * s.qt));
+  return s;
+}
+}  // namespace
+
+size_t umma_scratch_rows(const UmmaLeafArgs& a) {
+  const TcShape s = tc_shape(a);
+  int64_t leaves = a.leaves >> s.glog;
+  for (int t = 0; a.ftable && t < a.trees; ++t) leaves = std::max(leaves, a.fcount[t]);
+  return (size_t)std::min<int64_t>(kChunkRows, leaves * s.qtiles * (kBM * s.qt));
+}
+size_t umma_row_scratch_bytes() { return kCap * sizeof(uint2); }
+
 int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
-  const int Kp = ((a.d + kKC - 1) / kKC) * kKC;
-  if (Kp > 256 || a.kq > 32 || a.kq < a.k) return KNN_ERR_UNSUPPORTED;
+  const int nch = (a.d + kKC - 1) / kKC;
+  if (nch > 4 || a.kq > 32 || a.kq < a.k) return KNN_ERR_UNSUPPORTED;
   cudaStream_t st = a.stream;
   uint16_t* Xb = static_cast<uint16_t*>(a.Xb);
   // operand copy (FP16 EUCLIDEAN: the largest |x| first, for the row scale)
@@ -845,59 +1235,67 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
     k_max_abs<<<(unsigned)std::min<int64_t>((cnt + 255) / 256, 148 * 8), 256, 0, st>>>(a.X, cnt, a.maxabs);
     log.add();
   }
-  k_to_operand<<<(unsigned)((a.n * 32 + 255) / 256), 256, 0, st>>>(a.X, a.n, a.d, a.dpad, Kp, a.metric, a.f16,
+  const int ldr = umma_row_stride(a.d);
+  k_to_operand<<<(unsigned)((a.n * 32 + 255) / 256), 256, 0, st>>>(a.X, a.n, a.d, a.dpad, ldr, a.metric, a.f16,
                                                                     a.maxabs, a.norms, Xb, a.norms2);
   log.add();
-  const uint32_t idesc = idesc_for(a.f16);
-  const size_t smem = umma_smem_bytes(Kp);
+  CUtensorMap map;
+  if (!operand_map(a.Xp, a.n, ldr, a.f16, &map)) return KNN_ERR_CUDA;
   const int64_t leaves = a.leaves;
   // 2^glog sibling leaves per tile (the caller checks it is allowed)
-  const int glog = a.tc_group >= 4 ? 2 : a.tc_group == 2 ? 1 : 0;
+  const TcShape shape = tc_shape(a);
+  const int qt = shape.qt, glog = shape.glog;
   if (glog && (a.ftable || (a.maxleaf << glog) > kBM)) return KNN_ERR_UNSUPPORTED;
-  const int qtiles = glog ? 1 : (int)((a.maxleaf + kBM - 1) / kBM);
-  for (int t = 0; t < a.trees; ++t) {
-    const int32_t* perm = a.perm + (size_t)t * a.n;
-    const int64_t* ftab = a.ftable ? a.ftable + 4 * a.foff[t] : nullptr;
-    const int64_t tleaves = a.ftable ? a.fcount[t] : (leaves >> glog);
+  LeafTcArgs t{};
+  t.Xp = static_cast<const uint16_t*>(a.Xp);
+  t.np = a.np;
+  t.segs = a.segs;
+  t.akey = a.akey;
+  t.aid = a.aid;
+  t.err = a.err;
+  t.surv = static_cast<uint2*>(a.surv);
+  t.count = a.surv_count;
+  t.n = a.n;
+  t.idesc = idesc_for(a.f16);
+  t.ldr = ldr;
+  t.ksteps = (a.d + 15) / 16;
+  t.k = a.k;
+  t.kq = a.kq;
+  t.qtiles = shape.qtiles;
+  t.glog = glog;
+  const int units = ldr / 8;
+  for (int tr = 0; tr < a.trees; ++tr) {
+    t.perm = a.perm + (size_t)tr * a.n;
+    t.ftab = a.ftable ? a.ftable + 4 * a.foff[tr] : nullptr;
+    const int64_t tleaves = a.ftable ? a.fcount[tr] : (leaves >> glog);
     if (tleaves <= 0) {
       if (a.kev) {
-        cudaEventRecord(a.kev[2 * t], st);
-        cudaEventRecord(a.kev[2 * t + 1], st);
+        cudaEventRecord(a.kev[2 * tr], st);
+        cudaEventRecord(a.kev[2 * tr + 1], st);
       }
       continue;
     }
-    const unsigned grid = (unsigned)(tleaves * qtiles);
-    const int32_t* inv = nullptr;
-    if (t > 0 && a.inv && (a.ftable || a.maxblock > kBN)) {
-      k_inverse_order<<<(unsigned)std::min<int64_t>((a.n + 255) / 256, 148 * 16), 256, 0, st>>>(perm, a.n, a.inv);
-      log.add();
-      inv = a.inv;
-    }
-#define KNN_TC_LAUNCH_N(M, F, N)                                                                          \
-  do {                                                                                                    \
-    cudaFuncSetAttribute(k_leaf_tc<M, F, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-    k_leaf_tc<M, F, N><<<grid, kUThreads, smem, st>>>(Xb, idesc, a.segs, ftab, a.k, a.kq, qtiles, glog, perm, \
-                                                      inv, a.norms2, a.akey, a.aid, a.err);             \
-  } while (0)
-#define KNN_TC_LAUNCH(M, F)                    \
-  do {                                         \
-    if (Kp == 64) KNN_TC_LAUNCH_N(M, F, 1);    \
-    else if (Kp == 128) KNN_TC_LAUNCH_N(M, F, 2); \
-    else if (Kp == 192) KNN_TC_LAUNCH_N(M, F, 3); \
-    else KNN_TC_LAUNCH_N(M, F, 4);             \
-  } while (0)
-    if (a.kev) cudaEventRecord(a.kev[2 * t], st);
-    if (a.metric == KNN_METRIC_EUCLIDEAN) {
-      if (t == 0) KNN_TC_LAUNCH(KNN_METRIC_EUCLIDEAN, true);
-      else KNN_TC_LAUNCH(KNN_METRIC_EUCLIDEAN, false);
-    } else {
-      if (t == 0) KNN_TC_LAUNCH(KNN_METRIC_COSINE, true);
-      else KNN_TC_LAUNCH(KNN_METRIC_COSINE, false);
-    }
-    if (a.kev) cudaEventRecord(a.kev[2 * t + 1], st);
-#undef KNN_TC_LAUNCH
-#undef KNN_TC_LAUNCH_N
+    const int64_t blocks = tleaves * t.qtiles;
+    k_permute_operand<<<(unsigned)((a.n * units + 255) / 256), 256, 0, st>>>(
+        reinterpret_cast<const uint4*>(Xb), a.norms2, t.perm, a.n, units, static_cast<uint4*>(a.Xp), a.np);
     log.add();
+    if (tr > 0) {
+      const int32_t* inv = a.tree_inv ? a.tree_inv + (size_t)tr * a.n : a.inv;
+      if (!a.tree_inv) {
+        k_inverse_order<<<(unsigned)std::min<int64_t>((a.n + 255) / 256, 148 * 16), 256, 0, st>>>(t.perm, a.n, a.inv);
+        log.add();
+      }
+      k_list_positions<<<(unsigned)((a.n * a.kq + 255) / 256), 256, 0, st>>>(a.aid, t.perm, inv, a.n, a.kq, a.plist);
+      log.add();
+      t.plist = a.plist;
+    }
+    if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
+    const bool pre = tr < kPrepassTrees && a.maxleaf >= kPrepassMin;
+    if (a.metric == KNN_METRIC_EUCLIDEAN)
+      launch_tc_tree<KNN_METRIC_EUCLIDEAN>(tr, pre, qt, nch, map, t, blocks, st, log);
+    else
+      launch_tc_tree<KNN_METRIC_COSINE>(tr, pre, qt, nch, map, t, blocks, st, log);
+    if (a.kev) cudaEventRecord(a.kev[2 * tr + 1], st);
   }
   const size_t rsm = (size_t)8 * (a.dpad + 32 * 64 + 32) * sizeof(float);
   const unsigned rgrid = (unsigned)((a.n + 7) / 8);
