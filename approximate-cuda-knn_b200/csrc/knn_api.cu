@@ -562,11 +562,47 @@ int run_leaf_umma(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   return KNN_OK;
 }
 
+// Candidate filter of the propagation steps (H null: none).
+struct PropFilter {
+  void* H = nullptr;
+  float* delta = nullptr;
+  unsigned int* maxabs = nullptr;
+};
+
+// 16-bit rows for the steps that follow.  They take the tensor-core leaf
+// stage's operand buffer, which is done with by then and has the same size.
+int prepare_filter(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, int metric, const float* norms,
+                   cudaStream_t st, PropFilter* F, knn::LaunchLog& log) {
+  if (!knn::prop_filter_applies(k, d)) return KNN_OK;
+  knn::PropPrep a{};
+  a.X = X;
+  a.n = n;
+  a.d = d;
+  a.dpad = dpad;
+  a.metric = metric;
+  a.norms = norms;
+  a.stream = st;
+  int rc = C->get("Xp", (size_t)n * knn::prop_row_stride(d) * 2, &a.H);
+  if (!rc) rc = C->get("norms_perm", (size_t)n, &a.delta);
+  if (!rc) rc = C->get("maxabs", 1, &a.maxabs);
+  if (rc) return rc;
+  rc = knn::prop_prepare(a, log);
+  if (rc) return fail_cuda(cudaGetLastError(), "propagation rows launch");
+  F->H = a.H;
+  F->delta = a.delta;
+  F->maxabs = a.maxabs;
+  return KNN_OK;
+}
+
 int run_prop(const float* X, int64_t n, int d, int dpad, int k, int metric, const float* norms,
              const int32_t* order, Lists* L, bool with_flags, unsigned long long* counter,
-             cudaStream_t st, knn::LaunchLog& log, int warps = 0, const void* Xh = nullptr, int ldh = 0) {
+             cudaStream_t st, knn::LaunchLog& log, const PropFilter& F, int warps = 0, const void* Xh = nullptr,
+             int ldh = 0) {
   knn::PropArgs a{};
   a.X = X;
+  a.H = F.H;
+  a.delta = F.delta;
+  a.maxabs = F.maxabs;
   a.Xh = Xh;
   a.ldh = ldh;
   a.n = n;
@@ -637,7 +673,8 @@ int tune_leaf_tile(knn_context* C, const float* X, int64_t n, int d, int dpad, i
 }
 
 int tune_prop_warps(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, int metric,
-                    const float* norms, const int32_t* order, Lists* L, cudaStream_t st, int* best) {
+                    const float* norms, const int32_t* order, Lists* L, cudaStream_t st, const PropFilter& F,
+                    int* best) {
   const int cur = L->cur;
   float best_ms = 3.4e38f;
   *best = 0;
@@ -646,7 +683,7 @@ int tune_prop_warps(knn_context* C, const float* X, int64_t n, int d, int dpad, 
     for (int rep = 0; rep < 2; ++rep) {
       knn::LaunchLog tl;
       KNN_CK(cudaEventRecord(C->tev[0], st));
-      int rc = run_prop(X, n, d, dpad, k, metric, norms, order, L, true, nullptr, st, tl, w);
+      int rc = run_prop(X, n, d, dpad, k, metric, norms, order, L, true, nullptr, st, tl, F, w);
       L->cur = cur;  // the timing run's output is scratch
       if (!rc) rc = time_since(C, st, &ms);
       if (rc) return rc;
@@ -742,8 +779,8 @@ int pick_shapes(knn_context* C, const knn_options& o, bool may_tune, bool fp32_l
 
 int finish_prop_tuning(knn_context* C, const knn_options& o, const float* X, int64_t n, int d, int dpad, int k,
                        int metric, const float* norms, const int32_t* order, Lists* L, int64_t maxleaf,
-                       cudaStream_t st, Shapes* sh) {
-  int rc = tune_prop_warps(C, X, n, d, dpad, k, metric, norms, order, L, st, &sh->prop_warps);
+                       cudaStream_t st, const PropFilter& F, Shapes* sh) {
+  int rc = tune_prop_warps(C, X, n, d, dpad, k, metric, norms, order, L, st, F, &sh->prop_warps);
   if (rc) return rc;
   C->tuned[tune_key(metric, d, k, maxleaf)].second = sh->prop_warps;
   (void)o;
@@ -802,8 +839,10 @@ int learn_network(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   if (!rc)
     rc = run_leaf(C, Xs, ns, d, dpad, gk, kMlpGraphTrees, single_layout(ns, T.depth), metric, T.perm, norms, &L,
                   nullptr, st, log);
+  PropFilter F;
+  if (!rc) rc = prepare_filter(C, Xs, ns, d, dpad, gk, metric, norms, st, &F, log);
   for (int p = 0; !rc && p < kMlpGraphProps; ++p)
-    rc = run_prop(Xs, ns, d, dpad, gk, metric, norms, T.perm, &L, true, nullptr, st, log);
+    rc = run_prop(Xs, ns, d, dpad, gk, metric, norms, T.perm, &L, true, nullptr, st, log, F);
   if (rc) return rc;
   int32_t* graph = nullptr;
   float* gdist = nullptr;
@@ -1014,15 +1053,18 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
                   log, sh.leaf_tile, kev, sh.sparse, sh.pairs);
   }
   if (rc) return rc;
+  if (timed) KNN_CK(cudaEventRecord(C->ev[3], st));
+  PropFilter F;
+  if (props > 0) rc = prepare_filter(C, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+  if (rc) return rc;
   if (tune_prop) {
-    rc = finish_prop_tuning(C, o, P.X, n, d, P.dpad, k, metric, norms, T.perm, &L, lay.maxleaf, st, &sh);
+    rc = finish_prop_tuning(C, o, P.X, n, d, P.dpad, k, metric, norms, T.perm, &L, lay.maxleaf, st, F, &sh);
     if (rc) return rc;
   }
-  if (timed) KNN_CK(cudaEventRecord(C->ev[3], st));
 
   for (int p = 0; p < props; ++p) {
     rc = run_prop(P.X, n, d, P.dpad, k, metric, norms, T.perm, &L, true,
-                  stats ? counters + 2 + p : nullptr, st, log, sh.prop_warps, P.Xh, P.ldh);
+                  stats ? counters + 2 + p : nullptr, st, log, F, sh.prop_warps, P.Xh, P.ldh);
     if (rc) return rc;
   }
   if (timed) KNN_CK(cudaEventRecord(C->ev[4], st));
@@ -1211,13 +1253,16 @@ int group_compute(knn_context* C, const BatchGroup& g, int k, int trees, int pro
     rc = run_leaf(C, X, g.ntot, g.d, g.dpad, k, trees, lay, metric, T.perm, norms, &L, nullptr, st, log,
                   sh.leaf_tile, nullptr, sh.sparse, sh.pairs);
   if (rc) return rc;
+  if (stage_events) KNN_CK(cudaEventRecord(C->ev[3], st));
+  PropFilter F;
+  if (props > 0) rc = prepare_filter(C, X, g.ntot, g.d, g.dpad, k, metric, norms, st, &F, log);
+  if (rc) return rc;
   if (tune_prop) {
-    rc = finish_prop_tuning(C, o, X, g.ntot, g.d, g.dpad, k, metric, norms, T.perm, &L, lay.maxleaf, st, &sh);
+    rc = finish_prop_tuning(C, o, X, g.ntot, g.d, g.dpad, k, metric, norms, T.perm, &L, lay.maxleaf, st, F, &sh);
     if (rc) return rc;
   }
-  if (stage_events) KNN_CK(cudaEventRecord(C->ev[3], st));
   for (int p = 0; p < props; ++p) {
-    rc = run_prop(X, g.ntot, g.d, g.dpad, k, metric, norms, T.perm, &L, true, nullptr, st, log, sh.prop_warps);
+    rc = run_prop(X, g.ntot, g.d, g.dpad, k, metric, norms, T.perm, &L, true, nullptr, st, log, F, sh.prop_warps);
     if (rc) return rc;
   }
   if (stage_events) KNN_CK(cudaEventRecord(C->ev[4], st));
@@ -1615,7 +1660,10 @@ int knn_propagate_step(knn_context* ctx, const float* points, int64_t n, int32_t
   if (rc) return rc;
   KNN_CK(cudaMemcpyAsync(L.key[0], key_in, sizeof(float) * (size_t)n * k, cudaMemcpyHostToDevice, st));
   KNN_CK(cudaMemcpyAsync(L.id[0], idx_in, sizeof(int32_t) * (size_t)n * k, cudaMemcpyHostToDevice, st));
-  rc = run_prop(P.X, n, d, P.dpad, k, metric, norms, nullptr, &L, false, nullptr, st, log);
+  PropFilter F;
+  rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+  if (rc) return rc;
+  rc = run_prop(P.X, n, d, P.dpad, k, metric, norms, nullptr, &L, false, nullptr, st, log, F);
   if (rc) return rc;
   int32_t* di = nullptr;
   rc = ctx->get("out_idx", (size_t)n * k, &di);
@@ -1768,8 +1816,15 @@ int knn_propagate_range(knn_context* ctx, const void* points, int64_t n, int32_t
     knn::launch_norms(P.X, n, d, P.dpad, norms, st);
   }
   if (r1 > r0) {
+    // the filter's rows take one pass over all points: not for a small range
+    PropFilter F;
+    if ((r1 - r0) * 8 >= n) rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+    if (rc) return rc;
     knn::PropArgs a{};
     a.X = P.X;
+    a.H = F.H;
+    a.delta = F.delta;
+    a.maxabs = F.maxabs;
     a.Xh = P.Xh;
     a.ldh = P.ldh;
     a.n = n;

@@ -167,8 +167,26 @@ size_t umma_row_scratch_bytes();
 // Elements per row of the 16-bit operand copies: whole 16-byte units.
 inline int umma_row_stride(int d) { return (d + 7) & ~7; }
 
+// 16-bit rows for the propagation's candidate filter (propagate.cu).
+inline int prop_row_stride(int d) { return (d + 7) & ~7; }
+bool prop_filter_applies(int k, int d);
+struct PropPrep {
+  const float* X;
+  int64_t n;
+  int d, dpad, metric;
+  const float* norms;    // COSINE
+  void* H;               // out: [n][prop_row_stride(d)]
+  float* delta;          // out: [n]
+  unsigned int* maxabs;  // out: [1] (EUCLIDEAN, TAXICAB)
+  cudaStream_t stream;
+};
+int prop_prepare(const PropPrep& a, LaunchLog& log);
+
 struct PropArgs {
   const float* X;
+  const void* H;             // filter rows of prop_prepare with delta and maxabs, or null: every key exact
+  const float* delta;
+  const unsigned int* maxabs;
   const void* Xh;            // FP16 rows [n][ldh] (ldh % 8 == 0, zero padded), gathered instead of X; or null
   int ldh;
   int64_t n;
