@@ -385,6 +385,7 @@ int get_lists(knn_context* C, int64_t n, int k, Lists* L) {
 struct Layout {
   knn::SegView segs;
   int64_t leaves = 1, maxleaf = 1;
+  int64_t minleaf = 0;   // median trees: smallest leaf (the smallest leaf of n points is floor(n / 2^depth))
   int64_t maxblock = 0;  // bound on the points of a leaf block (0: unknown)
   int tc_group_max = 1;  // sibling leaves a tensor-core tile may hold (1, 2 or 4)
   bool own_blocks = false;  // every leaf holds k+1 points, so each leaf is its own block
@@ -435,13 +436,28 @@ Layout single_layout(int64_t n, int depth) {
   y.segs = knn::single_segment(n, 0, depth);
   y.leaves = int64_t(1) << depth;
   y.maxleaf = (n + y.leaves - 1) / y.leaves;
+  y.minleaf = n / y.leaves;
   return y;
+}
+
+// Whether the FP32 leaf stage goes through the tensor-core filter.  Six trees, dense
+// against filtered (ms): leaves of 80 points and more gain at every size (k = 8, d =
+// 64: 300 points, leaf 75, 0.44 against 0.38; 20,000, leaf 78, 1.20 against 0.84;
+// 200,000, leaf 97, 4.55 against 3.26; leaf 360, 9.7 against 3.0).  Smaller leaves
+// have little to reject, so it takes some rows to win back the launches (d = 64: 20,000 at leaf
+// 30 0.50 against 0.56, 40,000 at leaf 30 0.84 against 0.81), lists much shorter than a leaf
+// and rows short enough for a survivor's exact key to cost little more than a
+// dense tile's (200,000, leaf 49: k = 24, d = 128 4.88 against 4.62, d = 240 6.30 against 6.85).
+bool leaf_filter_applies(const Layout& lay, int64_t n, int d, int k, int metric) {
+  if (metric == KNN_METRIC_TAXICAB || d > 256 || k > 32 || !lay.own_blocks || lay.ftable || !lay.tree_inv) return false;
+  return lay.maxleaf >= 80 ||
+         (lay.maxleaf >= std::max(20, k + k / 2) && n * lay.maxleaf >= 800000 && d + 4 * k <= 256);
 }
 
 int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, int trees,
              const Layout& lay, int metric, const int32_t* perm, const float* norms, Lists* L,
              unsigned long long* counter, cudaStream_t st, knn::LaunchLog& log, int tile = 0,
-             cudaEvent_t* kev = nullptr, bool sparse = false, bool pairs = false) {
+             cudaEvent_t* kev = nullptr, bool sparse = false, bool pairs = false, bool filter_ok = false) {
   const int kw = (k + 31) / 32;
   knn::launch_init_lists(L->key[L->cur], L->id[L->cur], L->flags[L->cur], n, k, kw, st);
   log.add(2);
@@ -487,8 +503,62 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
     }
     if (rc) return rc;
   }
-  int rc = knn::leaf_stage(a, log);
+  const bool filter = filter_ok && leaf_filter_applies(lay, n, d, k, metric);
+  // A first tree has no lists to filter by, so all its pairs would survive: it takes
+  // dense tiles unless the bounding pass covers every leaf (six trees, 200,000 x 128,
+  // leaf 360: 3.8 ms with the first tree filtered, 5.9 without; leaf 250, where that
+  // pass does not apply: 15.8 against 6.5).
+  if (filter) a.trees = knn::umma_bounds_first_tree(lay.minleaf, k) ? 0 : 1;
+  int rc = a.trees > 0 ? knn::leaf_stage(a, log) : KNN_OK;
   if (rc) return fail_cuda(cudaGetLastError(), "leaf stage launch");
+  if (!filter || trees <= a.trees) return KNN_OK;
+  knn::FilterLeafArgs f{};
+  f.X = X;
+  f.n = n;
+  f.d = d;
+  f.dpad = dpad;
+  f.k = k;
+  f.trees = trees;
+  f.first_tree = a.trees;
+  f.metric = metric;
+  f.segs = lay.segs;
+  f.leaves = lay.leaves;
+  f.maxleaf = lay.maxleaf;
+  f.tc_group = lay.tc_group_max;
+  f.perm = perm;
+  f.tree_inv = lay.tree_inv;
+  f.norms = norms;
+  f.rkey = a.rkey;
+  f.rid = a.rid;
+  f.pair_counter = counter;
+  f.err = C->err_words;
+  f.kev = kev;
+  f.stream = st;
+  rc = C->get("Xp", (size_t)n * knn::umma_row_stride(d) * 2, &f.Xp);
+  if (!rc) rc = C->get("norms_perm", (size_t)n, &f.np);
+  if (!rc) rc = C->get("delta_perm", (size_t)n, &f.dp);
+  if (!rc) rc = C->get("plist", (size_t)n * k, &f.plist);
+  const size_t srows = knn::filter_scratch_rows(f);
+  if (!rc) rc = C->get("survivors", srows * knn::umma_row_scratch_bytes(), &f.surv);
+  if (!rc) rc = C->get("surv_count", srows, &f.count);
+  if (!rc) rc = C->get("maxabs", 1, &f.maxabs);
+  if (!rc) rc = C->get("leaf_survivors", (size_t)trees + 1, &f.survivors);
+  if (rc) return rc;
+  f.dense_tree = [&](int t, const unsigned long long* survivors, unsigned long long limit) {
+    knn::LeafArgs one = a;
+    one.first_tree = t;
+    one.trees = 1;
+    one.pairs = false;
+    one.guard = survivors;
+    one.guard_limit = limit;
+    one.kev = nullptr;
+    one.pair_counter = nullptr;  // the filter counts its pairs whichever way they are decided
+    one.dlist = nullptr;
+    one.tmask = nullptr;
+    return knn::leaf_stage(one, log);
+  };
+  rc = knn::leaf_stage_filtered(f, log);
+  if (rc) return fail_cuda(cudaGetLastError(), "filtered leaf stage launch");
   return KNN_OK;
 }
 
@@ -500,6 +570,10 @@ bool use_sparse_dims(const knn_options& o, int metric, const Layout& lay, int dp
   if (metric == KNN_METRIC_COSINE || lay.ftable || o.sparse_dims < 0 || dpad > 32767) return false;
   return o.sparse_dims > 0 || lay.maxleaf >= 1024;
 }
+
+// The tensor-core filter stands in for FP32 tiles unless the options ask for a
+// kind of tile.
+bool filter_allowed(const knn_options& o) { return o.leaf_tile == 0 && o.sparse_dims <= 0 && o.tile_pairs >= 0; }
 
 // Symmetric tile pairs (each key computed once for both of its points): on
 // unless the option turns them off, wherever every leaf is its own block.
@@ -1050,7 +1124,7 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
                        log, kev, sh.tc_group);
   } else {
     rc = run_leaf(C, P.X, n, d, P.dpad, k, trees, lay, metric, T.perm, norms, &L, stats ? counters : nullptr, st,
-                  log, sh.leaf_tile, kev, sh.sparse, sh.pairs);
+                  log, sh.leaf_tile, kev, sh.sparse, sh.pairs, filter_allowed(o));
   }
   if (rc) return rc;
   if (timed) KNN_CK(cudaEventRecord(C->ev[3], st));
@@ -1235,6 +1309,8 @@ int group_compute(knn_context* C, const BatchGroup& g, int k, int trees, int pro
   lay.segs = view;
   lay.leaves = g.leaves;
   lay.maxleaf = g.maxleaf;
+  lay.minleaf = g.ntot;
+  for (const auto& e : g.hsegs) lay.minleaf = std::min(lay.minleaf, e.n >> e.depth);
   lay.tree_inv = T.inv;
   for (const auto& e : g.hsegs) lay.maxblock = std::max(lay.maxblock, host_max_block(e.n, e.depth, k));
   lay.tc_group_max = tc_group_max(g.hsegs.data(), (int)g.hsegs.size(), k, g.maxleaf);
@@ -1251,7 +1327,7 @@ int group_compute(knn_context* C, const BatchGroup& g, int k, int trees, int pro
                        st, log, nullptr, sh.tc_group);
   else
     rc = run_leaf(C, X, g.ntot, g.d, g.dpad, k, trees, lay, metric, T.perm, norms, &L, nullptr, st, log,
-                  sh.leaf_tile, nullptr, sh.sparse, sh.pairs);
+                  sh.leaf_tile, nullptr, sh.sparse, sh.pairs, filter_allowed(o));
   if (rc) return rc;
   if (stage_events) KNN_CK(cudaEventRecord(C->ev[3], st));
   PropFilter F;

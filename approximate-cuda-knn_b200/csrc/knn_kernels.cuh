@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 #include "knn_internal.cuh"
@@ -105,6 +106,8 @@ struct LeafArgs {
   unsigned long long* pair_counter;  // optional
   int tile;              // 32 or 64 (0: 64): query x candidate tile, results identical
   int first_tree;        // trees [first_tree, first_tree + trees) of perm
+  const unsigned long long* guard;  // device word: one-sided tiles run only if it is above guard_limit (null: always)
+  unsigned long long guard_limit;
   cudaEvent_t* kev;      // [2 * trees] events around each tree's tile kernel, or null
   const int64_t* ftable;
   const int64_t* foff;
@@ -166,6 +169,41 @@ size_t umma_scratch_rows(const UmmaLeafArgs& a);  // from the shape fields
 size_t umma_row_scratch_bytes();
 // Elements per row of the 16-bit operand copies: whole 16-byte units.
 inline int umma_row_stride(int d) { return (d + 7) & ~7; }
+
+// FP32 leaf stage behind the tensor-core filter (leaf_umma.cu): EUCLIDEAN and
+// COSINE, d <= 256, k <= 32, median trees where every leaf is its own block.
+// Trees [first_tree, trees) are merged into the exact lists rkey / rid.
+struct FilterLeafArgs {
+  const float* X;
+  int64_t n;
+  int d, dpad, k, trees, first_tree, metric;
+  SegView segs;
+  int64_t leaves, maxleaf;
+  int tc_group;
+  const int32_t* perm;      // [trees][n]
+  const int32_t* tree_inv;  // [trees][n] inverse orders
+  const float* norms;       // COSINE
+  float* rkey;              // [n][k] in/out
+  uint32_t* rid;
+  void* Xp;                 // [n][umma_row_stride(d)] 16-bit scratch
+  float* np;                // [n] scratch
+  float* dp;                // [n] scratch
+  int32_t* plist;           // [n][k] scratch
+  void* surv;               // [filter_scratch_rows(...)][umma_row_scratch_bytes()] scratch
+  uint32_t* count;          // [filter_scratch_rows(...)] scratch
+  unsigned int* maxabs;
+  unsigned long long* survivors;  // [trees + 1] scratch: of each tree, after a zero
+  // launches tree t's dense tiles, which run if *survivors > limit
+  std::function<int(int t, const unsigned long long* survivors, unsigned long long limit)> dense_tree;
+  unsigned long long* pair_counter;
+  int* err;
+  cudaEvent_t* kev;
+  cudaStream_t stream;
+};
+// The bounding pass covers every leaf of at least minleaf points that is its own block.
+bool umma_bounds_first_tree(int64_t minleaf, int k);
+int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log);
+size_t filter_scratch_rows(const FilterLeafArgs& a);  // from the shape fields
 
 // 16-bit rows for the propagation's candidate filter (propagate.cu).
 inline int prop_row_stride(int d) { return (d + 7) & ~7; }

@@ -423,7 +423,9 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf(const float* _
                                               float* __restrict__ rkey, uint32_t* __restrict__ rid,
                                               unsigned long long* __restrict__ pair_counter,
                                               const int16_t* __restrict__ dlist,
-                                              const int32_t* __restrict__ dnch, int lmax) {
+                                              const int32_t* __restrict__ dnch, int lmax,
+                                              const unsigned long long* __restrict__ guard,
+                                              unsigned long long guard_limit) {
   constexpr int kTile = TILE;
   static_assert(TILE == 32 || TILE == 64, "tile of 32 or 64");
   __shared__ __align__(16) float Qs[kDC][TILE + 4];
@@ -432,6 +434,7 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf(const float* _
   __shared__ int32_t qid[kTile], cid[kTile];
   __shared__ float qnorm[kTile], cnorm[kTile];
 
+  if (guard && *guard <= guard_limit) return;
   // block = (leaf, query tile): the 64-row (or 32-row) query tiles of a large
   // leaf spread over gridDim.y, and each query row's list is read and written
   // by one block only
@@ -628,12 +631,14 @@ static int launch_leaf_tile(const LeafArgs& a, const int32_t* perm, const int64_
   }
   const int64_t qtiles = (a.maxleaf + TILE - 1) / TILE;
   dim3 grid((unsigned)leaves, (unsigned)std::min<int64_t>(qtiles, 65535));
+  if (a.guard)  // most of these launches return at once: no more blocks than fill the chip
+    grid.y = (unsigned)std::min<int64_t>(grid.y, (8 * 148 + leaves - 1) / leaves);
   if (kpl == 1)
-    k_leaf<METRIC, 1, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax);
+    k_leaf<METRIC, 1, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax, a.guard, a.guard_limit);
   else if (kpl == 2)
-    k_leaf<METRIC, 2, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax);
+    k_leaf<METRIC, 2, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax, a.guard, a.guard_limit);
   else
-    k_leaf<METRIC, 4, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax);
+    k_leaf<METRIC, 4, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax, a.guard, a.guard_limit);
   return 1;
 }
 

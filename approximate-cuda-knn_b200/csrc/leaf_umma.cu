@@ -66,6 +66,7 @@ constexpr int kCap = 192;
 constexpr int kFlushAt = kCap - kTN;  // a fuller buffer could not take another tile
 constexpr int kFlushMin = 24;         // rows merged along when one row's buffer is full
 constexpr int64_t kChunkRows = 1 << 19;  // rows (of whole blocks) per launch: bounds the survivor scratch
+constexpr uint32_t kOverflow = 0xFFFFFFFFu;  // FP32 filter: more survivors than the buffer holds, evaluate the block
 constexpr uint32_t kListed = 0x80000000u;  // count flag (first tree): the row's list was already written
 constexpr int kBand = 1024;           // block columns covered by the listed-column bitmap at a time
 constexpr int kBandWords = kBand / 32 + 1;
@@ -81,7 +82,7 @@ constexpr float kSlack = 4.76837158203125e-07f;  // 2^-21: filter widening, eigh
 // rows whose first leaf was poor, which alone cost more than the pass: integer
 // mixture as above, tiles 14.9 -> 12.7 ms; a third tree's pass gains nothing.
 constexpr int kPrepassTrees = 2;
-constexpr int kPrepassMin = 1024;
+constexpr int kPrepassMin = 256;
 constexpr int kGroups = 64;
 constexpr int kGS = kGroups + 1;
 // Shared memory of one epilogue warp: a slice's products and the bitmaps of
@@ -363,7 +364,20 @@ struct LeafTcArgs {
   SegView segs;
   uint32_t* akey;         // [n][kq] ordered keys
   uint32_t* aid;          // [n][kq]
-  uint2* surv;            // [blocks of the launch][128 QT][kCap] survivors: product, block column
+  // [blocks of the launch][128 QT][kCap] survivors: product (FP32 filter: unset, then the ordered exact key),
+  // block column (then the id)
+  uint2* surv;
+  // FP32 filter (BOUND)
+  const float* X;         // [n][dpad] FP32 rows
+  const float* norms;     // [n] FP32 norms (COSINE)
+  const float* dp;        // [n] bounds of the 16-bit rows' errors, in the tree's order
+  const float* rkey;      // [n][k] lists: exact keys
+  const unsigned int* maxabs;
+  unsigned long long* pair_counter;
+  unsigned long long* survivors;  // FP32 filter: [-1] of the tree before, [0] of this tree
+  unsigned long long survivor_limit;
+  float g, g1;            // FP32 rounding of a key; of a tile's sums
+  int d, dpad, metric;
   uint32_t* count;        // [blocks of the launch][128 QT] survivors of each row, kListed
   int64_t block0;         // first block of the launch
   int* err;
@@ -372,6 +386,42 @@ struct LeafTcArgs {
   int ldr, ksteps;        // row stride in elements; 16-element steps holding dims
   int k, kq, qtiles, glog;
 };
+
+// FP32 filter.  The 16-bit rows are s * (x - c) (COSINE: of the unit rows), c a
+// member row of the leaf, so that rounding errors scale with the leaf and not with
+// the data's offset; s is the power of two that brings the largest |x| of all
+// rows into [2^13, 2^14), so differences stay inside the FP16 range.
+__device__ __forceinline__ float bound_scale(const LeafTcArgs& a) {
+  if (a.metric == KNN_METRIC_COSINE) return 8192.f;
+  const float m = __uint_as_float(*a.maxabs);
+  if (!(m > 0.f && m < __int_as_float(0x7F800000))) return 1.f;
+  int e;
+  frexpf(m, &e);  // m in [2^(e-1), 2^e)
+  return ldexpf(1.f, max(-126, min(126, 14 - e)));
+}
+// A scaled distance that neither the pair of an exact key reaches nor any pair
+// with a smaller key.  Slack for what a key may lose to underflow of its squares
+// (EUCLIDEAN, d 2^-138), or for its rounding (COSINE: |u - v|^2 = 2 key, and the
+// dot product, both norms and the division round by less than 1.5 g in all).
+__device__ __forceinline__ float key_distance(float key, float scale, const LeafTcArgs& a) {
+  const float q = a.metric == KNN_METRIC_COSINE ? 2.f * fmaxf(key, 0.f) + 3.f * a.g : key + (float)a.d * 2.8698593e-42f;
+  return scale * __fsqrt_rn(q) * (1.f + a.g);
+}
+// The same for pairs of which only the 16-bit rows' squared distance (at most
+// sq) and error bounds are known.  Distances whose key overflows bound nothing.
+__device__ __forceinline__ float minimum_distance(float sq, float err, float scale, const LeafTcArgs& a) {
+  const float r = __fsqrt_rn(fmaxf(sq, 0.f)) + err;
+  const float slack = a.metric == KNN_METRIC_COSINE ? 6.f * a.g : (float)a.d * 5.7397186e-42f;
+  const float t = __fsqrt_rn(r * r + scale * (scale * slack)) * (1.f + 2.f * a.g);
+  return t < scale * 1.8e19f ? t : __int_as_float(0x7F800000);
+}
+
+// FP32 filter: whether dense tiles take the tree instead, by the survivors that
+// the tile kernel counted (tree: this one's; else the one before, whose answer
+// this one inherits).
+__device__ __forceinline__ bool too_many(const LeafTcArgs& a, int tree) {
+  return *reinterpret_cast<volatile unsigned long long*>(a.survivors + tree) > a.survivor_limit;
+}
 
 // Block b's leaf rows [lo, hi), candidate block [blo, bhi) (positions in the
 // tree's order) and first query row q0 of the leaf.
@@ -409,8 +459,9 @@ __device__ __forceinline__ BlockRange block_range(const LeafTcArgs& a, int64_t b
 // lists, kMergeRows rows at a time: every row's loads, sort and merge are
 // independent chains.  Lane r holds row r's id, norm, count and bound; surv the
 // rows' buffers (product, block column); np and perm start at the block.  Returns the
-// bounds, lowered to the new list tails.
-template <int METRIC>
+// bounds, lowered to the new list tails.  EXACT: the buffers hold ordered exact
+// keys and ids, the lists FP32 keys (+inf without id: empty).
+template <int METRIC, bool EXACT = false>
 __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, const float* np, const int32_t* perm,
                                                  int kq, const uint2* surv, int qid, float myn, int cnt, float tk,
                                                  uint32_t have, uint32_t rows) {
@@ -437,6 +488,7 @@ __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, 
       if (lane < kq && ((have >> r[i]) & 1u)) {
         lk[i] = akey[(size_t)id * kq + lane];
         li[i] = aid[(size_t)id * kq + lane];
+        if (EXACT) lk[i] = li[i] == kNoId ? kNoKey : orderable(__uint_as_float(lk[i]));
       }
     }
     for (int e0 = 0; e0 < most; e0 += 32) {
@@ -447,6 +499,11 @@ __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, 
         ci[i] = kNoId;
         if (e0 + lane < c[i]) {
           const uint2 v = surv[r[i] * kCap + e0 + lane];
+          if (EXACT) {
+            ck[i] = v.x;
+            ci[i] = v.y;
+            continue;
+          }
           const float dot = __uint_as_float(v.x);
           const uint32_t p = v.y;
           ck[i] = orderable(METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(xn, np[p]))
@@ -473,7 +530,8 @@ __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, 
     for (int i = 0; i < kMergeRows; ++i) {
       const int id = __shfl_sync(0xFFFFFFFFu, qid, r[i]);
       if (lane < kq) {
-        akey[(size_t)id * kq + lane] = lk[i];
+        akey[(size_t)id * kq + lane] =
+            !EXACT ? lk[i] : li[i] == kNoId ? 0x7F800000u : __float_as_uint(from_orderable(lk[i]));
         aid[(size_t)id * kq + lane] = li[i];
       }
       const float tail = from_orderable(__shfl_sync(0xFFFFFFFFu, lk[i], kq - 1));
@@ -501,7 +559,7 @@ __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, 
 // which bounds the rounding of both the key and the threshold.  A tail from an
 // earlier tile is looser than the current one, never tighter.  Every
 // survivor's exact key is computed at its merge and ranked there.
-template <int METRIC, bool FIRST, bool PRE, int NCH, int QT>
+template <int METRIC, bool BOUND, bool FIRST, bool PRE, int NCH, int QT>
 __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
     k_leaf_tc(const __grid_constant__ CUtensorMap bmap, const __grid_constant__ LeafTcArgs a) {
   using Plan = TmemPlan<NCH, QT>;
@@ -530,7 +588,9 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
   const int nb = (int)(bhi - blo);
   const int qts = min(QT, (nq - q0 + kBM - 1) / kBM);  // query tiles with rows
   const int nt = (nb + kTN - 1) / kTN;
-  const int npre = PRE && nb >= kPrepassMin && a.glog == 0 ? nt : 0;  // tiles of the bounding pass
+  // columns per group of the bounding pass, and its tiles: enough groups for the kq-th minimum
+  const int gw = nb <= 8 * kGroups ? 8 : nb <= 16 * kGroups ? 16 : 32;
+  const int npre = PRE && nb >= kPrepassMin && nb >= gw * (a.kq + a.kq / 4) && a.glog == 0 ? nt : 0;
   const int nsteps = npre + nt;
 
   if (warp == 4 * QT) {  // producer warp: barriers
@@ -549,8 +609,8 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
       }
       mbar_init(bar_done, 1);
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-      // an earlier block of the build gave up: do nothing
-      *status_p = *reinterpret_cast<volatile int*>(a.err) != 0 ? 2 : 0;
+      // an earlier block of the build gave up (or dense tiles take the tree): do nothing
+      *status_p = *reinterpret_cast<volatile int*>(a.err) != 0 || (BOUND && too_many(a, -1)) ? 2 : 0;
     }
     __syncwarp();
   } else if (warp == 4 * QT + 1) {  // MMA warp: tensor memory
@@ -573,6 +633,7 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
     const int64_t pos = lo + row;  // position in the tree's order
     const int qid = live ? a.perm[pos] : -1;
     const float myn = METRIC == KNN_METRIC_EUCLIDEAN && live ? a.np[pos] : 0.f;
+    const float mydl = BOUND && live ? a.dp[pos] : 0.f;
     if (!stopped && qt < qts) {
       // the row's 16-bit elements into tensor memory, two per 32-bit column
       const uint16_t* src = a.Xp + (size_t)(live ? pos : lo) * a.ldr;
@@ -620,8 +681,10 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
         ca = (int)(s - blo);
         cb = (int)(e - blo);
       }
-      float tk = kInf;          // bound on the row's kq-th key: its list tail, or the bounding pass's
-      float cm_all = 0.f;       // largest |y|^2 met in the bounding pass
+      // bound on the row's kq-th key (BOUND: scaled distance): its list tail, or the bounding pass's
+      float tk = kInf;
+      float cm_all = 0.f, dt_all = 0.f;  // largest |y|^2 and error bound met in the bounding pass
+      bool over = false;                 // BOUND: the buffer was too small
       int cnt = 0;              // buffered survivors
       uint32_t have = FIRST ? 0u : 0xFFFFFFFFu;  // rows whose list holds something
       // later trees: the bitmap, for every row, of the columns in [band, band + kBand)
@@ -644,8 +707,13 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
         }
         __syncwarp();
       };
+      const float scale = BOUND ? bound_scale(a) : 1.f;
       if (!FIRST) {
-        if (live) tk = from_orderable(a.akey[(size_t)qid * a.kq + a.kq - 1]);
+        if (BOUND) {
+          if (live) tk = key_distance(a.rkey[(size_t)qid * a.kq + a.kq - 1], scale, a);
+        } else {
+          if (live) tk = from_orderable(a.akey[(size_t)qid * a.kq + a.kq - 1]);
+        }
         if (!(tk < kInf)) tk = kInf;  // free slots
       }
       if (npre) {
@@ -668,8 +736,12 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const float* tn = tnorms + (s % kNormSlots) * (kTN + 4);
         const float cm = METRIC == KNN_METRIC_EUCLIDEAN ? tn[kTN] : 0.f;
+        const float dt = BOUND ? tn[kTN + 1] : 0.f;
         float thr = kMaxF;  // the row's filter bound
-        if (tk < kInf) {
+        if (BOUND) {
+          const float r = (tk + mydl + dt) * (1.f + a.g);
+          thr = fminf((r * r + a.g1 * (myn + cm)) - myn, kMaxF);  // inf: every column
+        } else if (tk < kInf) {
           if (METRIC == KNN_METRIC_EUCLIDEAN) thr = fminf((tk - myn) + kSlack * (fabsf(tk) + myn + cm), kMaxF);
           else thr = fminf((tk - 1.f) + kSlack * (fabsf(tk) + 2.f), kMaxF);
         }
@@ -699,35 +771,39 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
             // smallest key' of the slice, the row's own column and the columns
             // past the block left out, into the slice's group
             cm_all = fmaxf(cm_all, cm);
-            float m = kInf;
+            dt_all = fmaxf(dt_all, dt);
+            float big[4] = {-kInf, -kInf, -kInf, -kInf};  // of -key', per eight columns
             if (__any_sync(0xFFFFFFFFu, own >= 0 && own < 32) || lim < 32) {
 #pragma unroll
-              for (int c = 0; c < 32; ++c) {
-                const float kp = METRIC == KNN_METRIC_EUCLIDEAN
-                                     ? -__fmaf_rn(2.f, __uint_as_float(v[c]), tn[h * 32 + c])
-                                     : -__uint_as_float(v[c]);
-                m = c == own || c >= lim ? m : fminf(m, kp);
-              }
-            } else {
-              float big[4] = {-kInf, -kInf, -kInf, -kInf};
+              for (int c = 0; c < 32; ++c) v[c] = c == own || c >= lim ? 0xFF800000u : v[c];  // -inf: never the smallest
+            }
 #pragma unroll
-              for (int c = 0; c < 32; c += 4) {
-                uint32_t d[4] = {v[c], v[c + 1], v[c + 2], v[c + 3]};
-                if (METRIC == KNN_METRIC_EUCLIDEAN) {
-                  const ulonglong2 n = n4[c >> 2];
-                  unpack2(fma2(pack2(0x40000000u, 0x40000000u), pack2(d[0], d[1]), n.x), d[0], d[1]);
-                  unpack2(fma2(pack2(0x40000000u, 0x40000000u), pack2(d[2], d[3]), n.y), d[2], d[3]);
-                }
-                float& b0 = big[(c >> 1) & 3];
-                float& b1 = big[((c >> 1) & 3) + 1];
-                b0 = fmaxf(b0, fmaxf(__uint_as_float(d[0]), __uint_as_float(d[1])));
-                b1 = fmaxf(b1, fmaxf(__uint_as_float(d[2]), __uint_as_float(d[3])));
+            for (int c = 0; c < 32; c += 4) {
+              uint32_t d[4] = {v[c], v[c + 1], v[c + 2], v[c + 3]};
+              if (METRIC == KNN_METRIC_EUCLIDEAN) {
+                const ulonglong2 n = n4[c >> 2];
+                unpack2(fma2(pack2(0x40000000u, 0x40000000u), pack2(d[0], d[1]), n.x), d[0], d[1]);
+                unpack2(fma2(pack2(0x40000000u, 0x40000000u), pack2(d[2], d[3]), n.y), d[2], d[3]);
               }
-              m = -fmaxf(fmaxf(big[0], big[1]), fmaxf(big[2], big[3]));
+              float& b = big[c >> 3];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) b = fmaxf(b, __uint_as_float(d[e]));
             }
             norms_done();
-            float* group = gm + lane * kGS + ((2 * s + h) & (kGroups - 1));
-            *group = fminf(*group, m);
+            float* group = gm + lane * kGS;
+            const int slice = 2 * s + h;
+            if (gw == 32) {
+              float& x = group[slice & (kGroups - 1)];
+              x = fminf(x, -fmaxf(fmaxf(big[0], big[1]), fmaxf(big[2], big[3])));
+            } else if (gw == 16) {
+              float* x = group + ((2 * slice) & (kGroups - 1));
+              x[0] = fminf(x[0], -fmaxf(big[0], big[1]));
+              x[1] = fminf(x[1], -fmaxf(big[2], big[3]));
+            } else {
+              float* x = group + ((4 * slice) & (kGroups - 1));
+#pragma unroll
+              for (int e = 0; e < 4; ++e) x[e] = fminf(x[e], -big[e]);
+            }
             if (h == 1 && s == npre - 1) {
               // bound per row: the kq-th smallest of its group minima (kBoundRows
               // rows interleaved).  Each row's 64 minima: lanes' first halves sorted
@@ -775,7 +851,7 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
                 }
               }
               // key' -> key units, widened past the rounding of both
-              const float cap = METRIC == KNN_METRIC_EUCLIDEAN
+              const float cap = BOUND ? minimum_distance(bound + myn + a.g1 * (myn + cm_all), mydl + dt_all, scale, a) :  METRIC == KNN_METRIC_EUCLIDEAN
                                     ? (bound + myn) + kSlack * (fabsf(bound) + 2.f * myn + cm_all)
                                     : (bound + 1.f) + kSlack * (fabsf(bound) + 2.f);
               if (cap < tk) tk = cap;
@@ -816,7 +892,12 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
         }
             if (!FIRST) m &= ~bits[lane * kBandWords + (c0 % kBand) / 32];
             const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, m);
-            if (any) {
+            if (BOUND) {
+              if (any) {
+                over = over || cnt + __popc(m) > kCap;
+                for (uint32_t left = over ? 0u : m; left; left &= left - 1) mysurv[cnt++].y = (uint32_t)(c0 + __ffs(left) - 1);
+              }
+            } else if (any) {
               // the products through shared memory (a lane cannot index its registers);
               // then every lane appends its own survivors
 #pragma unroll
@@ -826,18 +907,22 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
                 const int c = __ffs(left) - 1;
                 mysurv[cnt++] = make_uint2(*reinterpret_cast<const uint32_t*>(dump + 4 * c), (uint32_t)(c0 + c));
               }
-        }
-        }
+            }
+          }
         }
         // a buffer too full for another tile is merged here (rare), with the
         // other well filled ones
-        if (pre || !__any_sync(0xFFFFFFFFu, cnt > kFlushAt)) continue;
+        if (BOUND || pre || !__any_sync(0xFFFFFFFFu, cnt > kFlushAt)) continue;
         const uint32_t rows = __ballot_sync(0xFFFFFFFFu, cnt >= kFlushMin);
         tk = merge_survivors<METRIC>(a.akey, a.aid, a.np + blo, a.perm + blo, a.kq, surv, qid, myn, cnt, tk, have, rows);
         have |= rows;
         if ((rows >> lane) & 1u) cnt = 0;
       }
-      if (ok) a.count[slot + lane] = (uint32_t)cnt | (FIRST && ((have >> lane) & 1u) ? kListed : 0u);
+      if (BOUND) {
+        const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, !ok ? 0u : over ? (uint32_t)nb : (uint32_t)cnt);
+        if (lane == 0 && sum) atomicAdd(a.survivors, (unsigned long long)sum);
+      }
+      if (ok) a.count[slot + lane] = BOUND && over ? kOverflow : (uint32_t)cnt | (FIRST && ((have >> lane) & 1u) ? kListed : 0u);
     }
   } else {
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -852,11 +937,12 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
       bool ok = true;
       // -|y|^2 of a tile's columns (EUCLIDEAN), -inf past the block, fetched a tile ahead
       const float kInf = __int_as_float(0x7F800000);
-      float f0 = 0.f, f1 = 0.f;
+      float f0 = 0.f, f1 = 0.f, e0 = 0.f;
       auto fetch_norms = [&](int s) {
         const int c = (s < npre ? s : s - npre) * kTN + lane;
         f0 = c < nb ? a.np[blo + c] : kInf;
         f1 = c + 32 < nb ? a.np[blo + c + 32] : kInf;
+        if (BOUND) e0 = fmaxf(c < nb ? a.dp[blo + c] : 0.f, c + 32 < nb ? a.dp[blo + c + 32] : 0.f);
       };
       if (METRIC == KNN_METRIC_EUCLIDEAN) fetch_norms(0);
       for (int s = 0; ok && s < nsteps; ++s) {
@@ -871,6 +957,10 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
           float* tn = tnorms + slot * (kTN + 4);
           tn[lane] = -f0;
           tn[lane + 32] = -f1;
+          if (BOUND) {
+            const uint32_t worst = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(e0));
+            if (lane == 0) tn[kTN + 1] = __uint_as_float(worst);
+          }
           // norms are >= 0, so their bit patterns order as unsigned integers
           const float fm = fmaxf(f0 < kInf ? f0 : 0.f, f1 < kInf ? f1 : 0.f);
           const uint32_t big = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(fm));
@@ -952,8 +1042,9 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
   }
 }
 
-// The survivors that k_leaf_tc left, into the lists: a warp takes 32 rows, the
-// rows with survivors (first tree: every row) kMergeRows at a time.  A kernel
+// The survivors that k_leaf_tc left, into the lists: a warp takes 32 rows (or an
+// equal part of them, by gridDim.y), the rows with survivors (first tree: every
+// row) kMergeRows at a time.  A kernel
 // of its own, so that sorting and merging run at full occupancy instead of in
 // the few warps that share an SM with the tiles, and never stall the products.
 template <int METRIC, bool FIRST, int QT>
@@ -961,7 +1052,7 @@ __global__ void __launch_bounds__(kBM * QT) k_leaf_tc_merge(const __grid_constan
   const BlockRange range = block_range<QT>(a, a.block0 + blockIdx.x);
   const int lane = threadIdx.x & 31;
   const int row = range.q0 + (int)threadIdx.x;
-  const bool live = row < (int)(range.hi - range.lo);
+  const bool live = row < (int)(range.hi - range.lo) && lane * (int)gridDim.y >> 5 == (int)blockIdx.y;
   if (*reinterpret_cast<volatile int*>(a.err) != 0) return;  // the build gave up: counts may be missing
   const size_t slot = (size_t)blockIdx.x * (kBM * QT) + threadIdx.x;
   uint32_t c = live ? a.count[slot] : 0u;
@@ -973,6 +1064,237 @@ __global__ void __launch_bounds__(kBM * QT) k_leaf_tc_merge(const __grid_constan
   const float myn = METRIC == KNN_METRIC_EUCLIDEAN && live ? a.np[pos] : 0.f;
   merge_survivors<METRIC>(a.akey, a.aid, a.np + range.blo, a.perm + range.blo, a.kq, a.surv + (slot - lane) * kCap,
                           qid, myn, (int)(c & ~kListed), 0.f, have, rows);
+}
+
+// FP32 filter: the exact key (the reference's order) of every survivor, into
+// the rows' lists.  A warp takes 32 rows (or an equal part of them, by gridDim.y)
+// and packs their survivors, a lane each:
+// the candidates' rows go through shared memory in slices (eight lanes read 128
+// contiguous bytes; wider slices when there are fewer of them), the queries' come
+// from L1.  Reading both straight from L1, a lane per survivor of one row, was
+// bound by L1's one line per cycle: 300,000 x 128, 16 trees, leaf 512, 6.8 ms against
+// 3.9.  A row whose buffer overflowed evaluates its whole block.
+constexpr int kExactPitch = 128 + 16;            // row pitch of a 32-dim slice
+constexpr int kExactBytes = 32 * kExactPitch;    // a warp's slice: 32 x 32, 16 x 64 or 8 x 128 dims
+template <int METRIC, int QT>
+__global__ void __launch_bounds__(kBM * QT, 10 / QT) k_leaf_tc_exact(const __grid_constant__ LeafTcArgs a,
+                                                            float* __restrict__ rkey, uint32_t* __restrict__ rid) {
+  __shared__ __align__(16) unsigned char slices[4 * QT * kExactBytes];
+  const BlockRange range = block_range<QT>(a, a.block0 + blockIdx.x);
+  const int lane = threadIdx.x & 31;
+  unsigned char* slice = slices + (threadIdx.x >> 5) * kExactBytes;
+  const int row = range.q0 + (int)threadIdx.x;
+  const bool live = row < (int)(range.hi - range.lo) && lane * (int)gridDim.y >> 5 == (int)blockIdx.y;
+  if (*reinterpret_cast<volatile int*>(a.err) != 0) return;  // the build gave up: counts may be missing
+  const float kInf = __int_as_float(0x7F800000);
+  const size_t slot = (size_t)blockIdx.x * (kBM * QT) + threadIdx.x;
+  const int64_t pos = range.lo + row;
+  if (a.pair_counter) {  // statistics: pairs the filter decided on
+    int64_t size = 0;
+    if (live) {
+      int64_t lo = range.lo, hi = range.hi;
+      if (a.glog) {  // the row's own leaf
+        for (int g = 0; g < (1 << a.glog); ++g) {
+          hi = range.seg.off + node_lo(range.seg.n, range.seg.depth, range.j + g + 1);
+          if (pos < hi) break;
+          lo = hi;
+        }
+      }
+      size = hi - lo - 1;
+    }
+    const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)size);
+    if (lane == 0 && sum) atomicAdd(a.pair_counter, (unsigned long long)sum);
+  }
+  if (too_many(a, 0)) return;  // dense tiles follow (a later chunk's count may still decide so: they repeat this one)
+  const uint32_t c = live ? a.count[slot] : 0u;
+  if (!__any_sync(0xFFFFFFFFu, c != 0u)) return;
+  const int qid = live ? a.perm[pos] : -1;
+  uint2* surv = a.surv + (slot - lane) * kCap;
+
+  // lane: the exact key of row r and the candidate at position p (valid lanes: the first m); cid: its id,
+  // tail: the row's list tail
+  auto keys = [&](int m, int r, int64_t p, int& cid, float& tail) {
+    const bool valid = lane < m;
+    const int id = __shfl_sync(0xFFFFFFFFu, qid, r);
+    cid = valid ? __ldg(a.perm + p) : 0;
+    tail = valid ? rkey[(size_t)id * a.k + a.k - 1] : -kInf;
+    const float4* xq = reinterpret_cast<const float4*>(a.X + (size_t)(valid ? id : 0) * a.dpad);
+    const int wlog = m <= 8 ? 7 : m <= 16 ? 6 : 5, width = 1 << wlog, pitch = 4 * width + 16;
+    const int ulog = wlog - 2, c1 = lane & ((1 << ulog) - 1), r1 = lane >> ulog, rstep = 32 >> ulog;
+    float total = 0.f, part = 0.f;
+    for (int cd = 0; cd < a.d; cd += width) {
+      const int dim = cd + 4 * c1;
+      for (int i0 = 0; i0 < m; i0 += rstep) {
+        const int i = i0 + r1;
+        const int cand = __shfl_sync(0xFFFFFFFFu, cid, i & 31);
+        if (i < m)
+          cp_async16(smem_u32(slice + i * pitch + c1 * 16), a.X + (size_t)cand * a.dpad + (dim < a.dpad ? dim : 0),
+                     dim < a.dpad ? 16 : 0);
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncwarp();
+      if (valid) {
+        const float4* mine = reinterpret_cast<const float4*>(slice + lane * pitch);
+        const int nu = (min(width, a.d - cd) + 3) / 4;
+#pragma unroll 8
+        for (int u = 0; u < nu; ++u) {
+          const float4 w = mine[u];
+          const float4 v = __ldg(xq + (cd >> 2) + u);
+          part = acc_step<METRIC>(v.x, w.x, part);
+          part = acc_step<METRIC>(v.y, w.y, part);
+          part = acc_step<METRIC>(v.z, w.z, part);
+          part = acc_step<METRIC>(v.w, w.w, part);
+        }
+        if (((cd + width) & 255) == 0 || cd + width >= a.d) {
+          total = __fadd_rn(total, part);
+          part = 0.f;
+        }
+      }
+      __syncwarp();  // the slice is refilled next
+    }
+    float key = total;
+    if (METRIC == KNN_METRIC_COSINE && valid) key = cosine_key(total, a.norms[id], a.norms[cid]);
+    return key;
+  };
+
+  // the rows' survivors side by side: lane r holds the first slot of row r
+  const int mine = c == kOverflow ? 0 : (int)c;
+  int first = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xFFFFFFFFu, first, o);
+    if (lane >= o) first += v;
+  }
+  const int all = __shfl_sync(0xFFFFFFFFu, first, 31);
+  first -= mine;
+  for (int e0 = 0; e0 < all; e0 += 32) {
+    const int e = min(e0 + lane, all - 1);
+    int r = 0;  // the last row whose first slot is at most e
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1)
+      if (__shfl_sync(0xFFFFFFFFu, first, r + o) <= e) r += o;
+    uint2* at = surv + (size_t)r * kCap + (e - __shfl_sync(0xFFFFFFFFu, first, r));
+    int cid;
+    float tail;
+    const float key = keys(min(32, all - e0), r, range.blo + at->y, cid, tail);
+    // the survivor's key and id take its place
+    if (e0 + lane < all) *at = key <= tail ? make_uint2(orderable(key), (uint32_t)cid) : make_uint2(kNoKey, kNoId);
+  }
+  uint32_t rows = __ballot_sync(0xFFFFFFFFu, mine > 0);
+  if (rows)
+    merge_survivors<METRIC, true>(reinterpret_cast<uint32_t*>(rkey), rid, nullptr, nullptr, a.k, surv, qid, 0.f, mine,
+                                  0.f, 0xFFFFFFFFu, rows);
+  // overflowed rows: every column of the block
+  for (rows = __ballot_sync(0xFFFFFFFFu, c == kOverflow); rows; rows &= rows - 1) {
+    const int nb = (int)(range.bhi - range.blo), r = __ffs(rows) - 1;
+    const int id = __shfl_sync(0xFFFFFFFFu, qid, r);
+    WarpList<1> L;
+    L.key[0] = lane < a.k ? rkey[(size_t)id * a.k + lane] : kInf;
+    L.id[0] = lane < a.k ? rid[(size_t)id * a.k + lane] : kNoId;
+    for (int e0 = 0; e0 < nb; e0 += 32) {
+      int cid;
+      float tk;
+      uint32_t ti;
+      const float key = keys(min(32, nb - e0), r, range.blo + min(e0 + lane, nb - 1), cid, tk);
+      warp_list_get(L, a.k - 1, tk, ti);
+      bool pass = e0 + lane < nb && cid != id && cand_less(key, (uint32_t)cid, tk, ti);
+      if (!__any_sync(0xFFFFFFFFu, pass)) continue;
+      const bool dup = warp_list_contains(L, (uint32_t)cid, a.k);
+      pass = pass && !dup;
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, pass);
+      if (bal) warp_list_insert_lanes(L, bal, key, (uint32_t)cid, kInf);
+    }
+    if (lane < a.k) {
+      rkey[(size_t)id * a.k + lane] = L.key[0];
+      rid[(size_t)id * a.k + lane] = L.id[0];
+    }
+    __syncwarp();
+  }
+}
+
+// FP32 filter: a tree's 16-bit rows (see bound_scale): Xp = fp16(s (x - c)), np =
+// |row|^2, dp bounds |s (x - c) - row| (L2).  A row that defeats the bound (a COSINE
+// norm whose square leaves the FP32 range or is zero) becomes a zero row with dp =
+// inf: always a survivor.  Infinite values and NaN, which have keys that no order
+// ranks, leave the tree to the dense tiles.  Bound by the gather of the
+// rows: a warp takes kCenterRows positions, whose leaves its lanes look up side by side.
+constexpr int kCenterRows = 8;
+__global__ void __launch_bounds__(256) k_center_operand(const __grid_constant__ LeafTcArgs a, uint16_t* __restrict__ Xp,
+                                                        float* __restrict__ np, float* __restrict__ dp) {
+  const int64_t p0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kCenterRows;
+  const int lane = threadIdx.x & 31;
+  if (too_many(a, -1)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.survivors[0] = a.survivors[-1];
+    return;
+  }
+  if (p0 >= a.n) return;
+  const float scale = bound_scale(a);
+  int32_t my_id = 0, my_cid = 0;
+  float my_rx = 1.f, my_rc = 1.f;
+  bool my_ok = true;
+  if (lane < kCenterRows && p0 + lane < a.n) {
+    const int64_t p = p0 + lane;
+    const SegEntry e = a.segs.get(a.segs.of(p));
+    const int64_t j = node_of(e.n, e.depth, p - e.off);
+    const int64_t mid = e.off + (node_lo(e.n, e.depth, j) + node_lo(e.n, e.depth, j + 1)) / 2;
+    my_id = __ldg(a.perm + p);
+    my_cid = __ldg(a.perm + mid);
+    if (a.metric == KNN_METRIC_COSINE) {
+      const float nx = a.norms[my_id], nc = a.norms[my_cid];
+      my_ok = nx > 8.67361738e-19f && nx < 1.15292150e18f;  // 2^-60, 2^60
+      my_rx = __frcp_rn(nx);  // 0 or NaN: not finite
+      my_rc = nc > 8.67361738e-19f && nc < 1.15292150e18f ? __frcp_rn(nc) : 0.f;
+    }
+  }
+  const float base = a.metric == KNN_METRIC_COSINE ? scale * 4.76837158e-07f : 0.f;  // 2^-21: rounding of both unit rows
+  const int rows = (int)min((int64_t)kCenterRows, a.n - p0);
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    const int32_t id = __shfl_sync(0xFFFFFFFFu, my_id, r), cid = __shfl_sync(0xFFFFFFFFu, my_cid, r);
+    const float rx = __shfl_sync(0xFFFFFFFFu, my_rx, r), rc = __shfl_sync(0xFFFFFFFFu, my_rc, r);
+    const float4* x4 = reinterpret_cast<const float4*>(a.X + (size_t)id * a.dpad);
+    const float4* c4 = reinterpret_cast<const float4*>(a.X + (size_t)cid * a.dpad);
+    uint16_t* out = Xp + (size_t)(p0 + r) * a.ldr;
+    float err = 0.f, sq = 0.f;
+    for (int i = 4 * lane; i < a.ldr; i += 128) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f), c = x;  // rows are zero padded to dpad
+      if (i < a.dpad) {
+        x = __ldg(x4 + (i >> 2));
+        c = __ldg(c4 + (i >> 2));
+      }
+      const float v[4] = {__fmul_rn(__fsub_rn(__fmul_rn(x.x, rx), __fmul_rn(c.x, rc)), scale),
+                          __fmul_rn(__fsub_rn(__fmul_rn(x.y, rx), __fmul_rn(c.y, rc)), scale),
+                          __fmul_rn(__fsub_rn(__fmul_rn(x.z, rx), __fmul_rn(c.z, rc)), scale),
+                          __fmul_rn(__fsub_rn(__fmul_rn(x.w, rx), __fmul_rn(c.w, rc)), scale)};
+      uint32_t h[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const __half y = __float2half_rn(v[q]);
+        h[q] = __half_as_ushort(y);
+        const float f = __half2float(y), t = __fsub_rn(v[q], f);
+        err = __fmaf_rn(t, t, err);
+        sq = __fmaf_rn(f, f, sq);
+      }
+      *reinterpret_cast<uint2*>(out + i) = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+    }
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+      err = __fadd_rn(err, __shfl_xor_sync(0xFFFFFFFFu, err, off));
+      sq = __fadd_rn(sq, __shfl_xor_sync(0xFFFFFFFFu, sq, off));
+    }
+    // the subtraction's own rounding: 2^-23 of the row
+    const float bound = __fsqrt_rn(err) * (1.f + 1.f / 1024.f) + __fsqrt_rn(sq) * 1.1920929e-07f + base;
+    const bool usable = __shfl_sync(0xFFFFFFFFu, my_ok ? 1 : 0, r) != 0;
+    const bool good = usable && bound < __int_as_float(0x7F800000) && sq < __int_as_float(0x7F800000);
+    if (!good)
+      for (int i = 4 * lane; i < a.ldr; i += 128) *reinterpret_cast<uint2*>(out + i) = make_uint2(0u, 0u);
+    if (lane == 0) {
+      if (!(rx > 0.f) || (usable && !good)) atomicMax(a.survivors, a.survivor_limit + 1ull);
+      np[p0 + r] = good ? sq : 0.f;
+      dp[p0 + r] = good ? bound : __int_as_float(0x7F800000);
+    }
+  }
 }
 
 // inv[order[i]] = i: the position of each point in a tree's order.
@@ -1163,35 +1485,48 @@ bool operand_map(const void* Xp, int64_t n, int ldr, bool f16, CUtensorMap* map)
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A tree's tiles, kChunkRows rows at a time, each chunk followed by its merge.
-template <int METRIC, bool FIRST, bool PRE, int NCH, int QT>
-void launch_tc(const CUtensorMap& map, LeafTcArgs t, int64_t blocks, cudaStream_t st, LaunchLog& log) {
+// A tree's tiles, kChunkRows rows at a time, each chunk followed by its merge
+// (BOUND: into the exact lists rkey / rid).
+template <int METRIC, bool BOUND, bool FIRST, bool PRE, int NCH, int QT>
+void launch_tc(const CUtensorMap& map, LeafTcArgs t, int64_t blocks, float* rkey, uint32_t* rid, cudaStream_t st,
+               LaunchLog& log) {
   const size_t smem = leaf_tc_smem<NCH, QT>();
-  cudaFuncSetAttribute(k_leaf_tc<METRIC, FIRST, PRE, NCH, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k_leaf_tc<METRIC, BOUND, FIRST, PRE, NCH, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem);
   const int64_t chunk = kChunkRows / (kBM * QT);
   for (t.block0 = 0; t.block0 < blocks; t.block0 += chunk) {
     const unsigned grid = (unsigned)std::min(chunk, blocks - t.block0);
-    k_leaf_tc<METRIC, FIRST, PRE, NCH, QT><<<grid, 64 + 128 * QT, smem, st>>>(map, t);
-    k_leaf_tc_merge<METRIC, FIRST, QT><<<grid, kBM * QT, 0, st>>>(t);
+    k_leaf_tc<METRIC, BOUND, FIRST, PRE, NCH, QT><<<grid, 64 + 128 * QT, smem, st>>>(map, t);
+    // Few rows leave most of the chip idle in the kernels after the tiles, where a
+    // warp works through its 32 rows' survivors at the latency of its loads: each
+    // warp's rows are spread over up to eight warps until 8,000 are there (a chip
+    // holds 5,920; FP32, 36,155 x 246, 11 trees, leaf 104: one warp 4.09 ms, two 3.07,
+    // four 2.68, eight 2.56; 300,000 x 128, 16 trees, leaf 512: 10.78, 10.81, 11.30,
+    // 12.38; BF16 products, 5,206 x 23, 5 trees, leaf 77: 0.45, 0.39, 0.37, 0.35).
+    dim3 split(grid, 1);
+    while (split.y < 8 && 4 * QT * grid * split.y < 8000) split.y *= 2;
+    if (!BOUND) k_leaf_tc_merge<METRIC, FIRST, QT><<<split, kBM * QT, 0, st>>>(t);
+    else if (t.metric == KNN_METRIC_COSINE) k_leaf_tc_exact<KNN_METRIC_COSINE, QT><<<split, kBM * QT, 0, st>>>(t, rkey, rid);
+    else k_leaf_tc_exact<KNN_METRIC_EUCLIDEAN, QT><<<split, kBM * QT, 0, st>>>(t, rkey, rid);
     log.add(2);
   }
 }
-template <int METRIC, bool FIRST, bool PRE>
-void launch_tc_tiles(int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks, cudaStream_t st,
-                     LaunchLog& log) {
-  if (qt == 2 && nch == 1) launch_tc<METRIC, FIRST, PRE, 1, 2>(map, t, blocks, st, log);
-  else if (qt == 2) launch_tc<METRIC, FIRST, PRE, 2, 2>(map, t, blocks, st, log);
-  else if (nch == 1) launch_tc<METRIC, FIRST, PRE, 1, 1>(map, t, blocks, st, log);
-  else if (nch == 2) launch_tc<METRIC, FIRST, PRE, 2, 1>(map, t, blocks, st, log);
-  else if (nch == 3) launch_tc<METRIC, FIRST, PRE, 3, 1>(map, t, blocks, st, log);
-  else launch_tc<METRIC, FIRST, PRE, 4, 1>(map, t, blocks, st, log);
+template <int METRIC, bool BOUND, bool FIRST, bool PRE>
+void launch_tc_tiles(int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks, float* rkey,
+                     uint32_t* rid, cudaStream_t st, LaunchLog& log) {
+  if (qt == 2 && nch == 1) launch_tc<METRIC, BOUND, FIRST, PRE, 1, 2>(map, t, blocks, rkey, rid, st, log);
+  else if (qt == 2) launch_tc<METRIC, BOUND, FIRST, PRE, 2, 2>(map, t, blocks, rkey, rid, st, log);
+  else if (nch == 1) launch_tc<METRIC, BOUND, FIRST, PRE, 1, 1>(map, t, blocks, rkey, rid, st, log);
+  else if (nch == 2) launch_tc<METRIC, BOUND, FIRST, PRE, 2, 1>(map, t, blocks, rkey, rid, st, log);
+  else if (nch == 3) launch_tc<METRIC, BOUND, FIRST, PRE, 3, 1>(map, t, blocks, rkey, rid, st, log);
+  else launch_tc<METRIC, BOUND, FIRST, PRE, 4, 1>(map, t, blocks, rkey, rid, st, log);
 }
-template <int METRIC>
-void launch_tc_tree(int tree, bool pre, int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks,
-                    cudaStream_t st, LaunchLog& log) {
-  if (tree == 0) launch_tc_tiles<METRIC, true, true>(qt, nch, map, t, blocks, st, log);
-  else if (pre) launch_tc_tiles<METRIC, false, true>(qt, nch, map, t, blocks, st, log);
-  else launch_tc_tiles<METRIC, false, false>(qt, nch, map, t, blocks, st, log);
+template <int METRIC, bool BOUND>
+void launch_tc_tree(bool first, bool pre, int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks,
+                    float* rkey, uint32_t* rid, cudaStream_t st, LaunchLog& log) {
+  if (first) launch_tc_tiles<METRIC, BOUND, true, true>(qt, nch, map, t, blocks, rkey, rid, st, log);
+  else if (pre) launch_tc_tiles<METRIC, BOUND, false, true>(qt, nch, map, t, blocks, rkey, rid, st, log);
+  else launch_tc_tiles<METRIC, BOUND, false, false>(qt, nch, map, t, blocks, rkey, rid, st, log);
 }
 
 }  // namespace
@@ -1206,17 +1541,17 @@ namespace {
 struct TcShape {
   int qt, qtiles, glog;
 };
-TcShape tc_shape(const UmmaLeafArgs& a) {
+TcShape tc_shape(int d, int64_t maxleaf, int tc_group) {
   TcShape s;
-  s.glog = a.tc_group >= 4 ? 2 : a.tc_group == 2 ? 1 : 0;
-  s.qt = a.d > 2 * kKC || s.glog || a.maxleaf <= kBM ? 1 : 2;
-  s.qtiles = s.glog ? 1 : (int)((a.maxleaf + kBM * s.qt - 1) / (kBM * s.qt));
+  s.glog = tc_group >= 4 ? 2 : tc_group == 2 ? 1 : 0;
+  s.qt = d > 2 * kKC || s.glog || maxleaf <= kBM ? 1 : 2;
+  s.qtiles = s.glog ? 1 : (int)((maxleaf + kBM * s.qt - 1) / (kBM * s.qt));
   return s;
 }
 }  // namespace
 
 size_t umma_scratch_rows(const UmmaLeafArgs& a) {
-  const TcShape s = tc_shape(a);
+  const TcShape s = tc_shape(a.d, a.maxleaf, a.tc_group);
   int64_t leaves = a.leaves >> s.glog;
   for (int t = 0; a.ftable && t < a.trees; ++t) leaves = std::max(leaves, a.fcount[t]);
   return (size_t)std::min<int64_t>(kChunkRows, leaves * s.qtiles * (kBM * s.qt));
@@ -1243,7 +1578,7 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
   if (!operand_map(a.Xp, a.n, ldr, a.f16, &map)) return KNN_ERR_CUDA;
   const int64_t leaves = a.leaves;
   // 2^glog sibling leaves per tile (the caller checks it is allowed)
-  const TcShape shape = tc_shape(a);
+  const TcShape shape = tc_shape(a.d, a.maxleaf, a.tc_group);
   const int qt = shape.qt, glog = shape.glog;
   if (glog && (a.ftable || (a.maxleaf << glog) > kBM)) return KNN_ERR_UNSUPPORTED;
   LeafTcArgs t{};
@@ -1292,9 +1627,9 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
     if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
     const bool pre = tr < kPrepassTrees && a.maxleaf >= kPrepassMin;
     if (a.metric == KNN_METRIC_EUCLIDEAN)
-      launch_tc_tree<KNN_METRIC_EUCLIDEAN>(tr, pre, qt, nch, map, t, blocks, st, log);
+      launch_tc_tree<KNN_METRIC_EUCLIDEAN, false>(tr == 0, pre, qt, nch, map, t, blocks, nullptr, nullptr, st, log);
     else
-      launch_tc_tree<KNN_METRIC_COSINE>(tr, pre, qt, nch, map, t, blocks, st, log);
+      launch_tc_tree<KNN_METRIC_COSINE, false>(tr == 0, pre, qt, nch, map, t, blocks, nullptr, nullptr, st, log);
     if (a.kev) cudaEventRecord(a.kev[2 * tr + 1], st);
   }
   const size_t rsm = (size_t)8 * (a.dpad + 32 * 64 + 32) * sizeof(float);
@@ -1307,6 +1642,84 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
     k_rerank<KNN_METRIC_COSINE><<<rgrid, 256, rsm, st>>>(a.X, a.n, a.d, a.dpad, a.k, a.kq, a.norms, a.aid, a.rkey, a.rid);
   }
   log.add();
+  return cudaPeekAtLastError() == cudaSuccess ? KNN_OK : KNN_ERR_CUDA;
+}
+
+// ---------------------------------------------------------- FP32 leaf filter --
+size_t filter_scratch_rows(const FilterLeafArgs& a) {
+  const TcShape s = tc_shape(a.d, a.maxleaf, a.tc_group);
+  return (size_t)std::min<int64_t>(kChunkRows, (a.leaves >> s.glog) * s.qtiles * (kBM * s.qt));
+}
+
+// Group widths of 8, 16 and 32 start at 256, 513 and 1,025 columns, so groups times
+// width reach 1.25 k at every size from minleaf on if they do at 256.
+bool umma_bounds_first_tree(int64_t minleaf, int k) { return minleaf >= kPrepassMin && 8 * (k + k / 4) <= kPrepassMin; }
+
+int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
+  const int nch = (a.d + kKC - 1) / kKC;
+  if (nch > 4 || a.k > 32 || a.metric == KNN_METRIC_TAXICAB) return KNN_ERR_UNSUPPORTED;
+  cudaStream_t st = a.stream;
+  const TcShape shape = tc_shape(a.d, a.maxleaf, a.tc_group);
+  const int ldr = umma_row_stride(a.d);
+  if (a.metric == KNN_METRIC_EUCLIDEAN) {
+    cudaMemsetAsync(a.maxabs, 0, sizeof(unsigned int), st);
+    const int64_t cnt = a.n * (int64_t)a.dpad;
+    k_max_abs<<<(unsigned)std::min<int64_t>((cnt + 255) / 256, 148 * 8), 256, 0, st>>>(a.X, cnt, a.maxabs);
+    log.add();
+  }
+  CUtensorMap map;
+  if (!operand_map(a.Xp, a.n, ldr, true, &map)) return KNN_ERR_CUDA;
+  LeafTcArgs t{};
+  t.Xp = static_cast<const uint16_t*>(a.Xp);
+  t.np = a.np;
+  t.dp = a.dp;
+  t.segs = a.segs;
+  t.aid = a.rid;
+  t.err = a.err;
+  t.n = a.n;
+  t.idesc = idesc_for(true);
+  t.ldr = ldr;
+  t.ksteps = (a.d + 15) / 16;
+  t.k = t.kq = a.k;
+  t.qtiles = shape.qtiles;
+  t.glog = shape.glog;
+  t.surv = static_cast<uint2*>(a.surv);
+  t.count = a.count;
+  t.X = a.X;
+  t.norms = a.norms;
+  t.rkey = a.rkey;
+  t.maxabs = a.maxabs;
+  t.pair_counter = a.pair_counter;
+  t.g = (float)(2 * a.d + 64) * 5.9604644775390625e-08f;   // 2^-24
+  t.g1 = (float)(a.d + 64) * 4.76837158203125e-07f;        // 2^-21: the tensor cores' sums are not rounded to nearest
+  t.d = a.d;
+  t.dpad = a.dpad;
+  t.metric = a.metric;
+  const int64_t blocks = (a.leaves >> shape.glog) * shape.qtiles;
+  // Data that the 16-bit rows cannot tell apart (several scales within one leaf)
+  // would send most pairs down the survivors' path, at several times a dense
+  // tile's cost (400,000 x 256, leaf 1,000, all pairs: 415 ms against 64), so from
+  // an eighth of the pairs and 16 + k a row the dense tiles take over.
+  cudaMemsetAsync(a.survivors, 0, sizeof(unsigned long long) * (size_t)(a.trees + 1), st);
+  t.survivor_limit = (unsigned long long)a.n * (unsigned long long)(16 + a.k + a.maxleaf / 8);
+  for (int tr = a.first_tree; tr < a.trees; ++tr) {
+    if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
+    t.perm = a.perm + (size_t)tr * a.n;
+    t.survivors = a.survivors + tr + 1;
+    k_center_operand<<<(unsigned)((a.n + 8 * kCenterRows - 1) / (8 * kCenterRows)), 256, 0, st>>>(t, static_cast<uint16_t*>(a.Xp), a.np, a.dp);
+    log.add();
+    if (tr > 0) {
+      k_list_positions<<<(unsigned)((a.n * a.k + 255) / 256), 256, 0, st>>>(a.rid, t.perm, a.tree_inv + (size_t)tr * a.n,
+                                                                            a.n, a.k, a.plist);
+      log.add();
+      t.plist = a.plist;
+    }
+    const bool pre = tr < kPrepassTrees && a.maxleaf >= kPrepassMin;
+    launch_tc_tree<KNN_METRIC_EUCLIDEAN, true>(tr == 0, pre, shape.qt, nch, map, t, blocks, a.rkey, a.rid, st, log);
+    const int rc = a.dense_tree(tr, t.survivors, t.survivor_limit);
+    if (rc) return rc;
+    if (a.kev) cudaEventRecord(a.kev[2 * tr + 1], st);
+  }
   return cudaPeekAtLastError() == cudaSuccess ? KNN_OK : KNN_ERR_CUDA;
 }
 
