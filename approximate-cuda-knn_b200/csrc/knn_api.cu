@@ -1778,7 +1778,8 @@ int knn_exact_fp64(knn_context* ctx, const void* points, int64_t n, int32_t d, i
   int dev_sms = 148;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int64_t qtiles = (nq + 63) / 64;
-  int slices = (int)((4LL * dev_sms + qtiles - 1) / qtiles);
+  // two whole waves of two blocks per SM, never a third wave of a few blocks
+  int slices = (int)((4LL * dev_sms) / qtiles);
   if (slices < 1) slices = 1;
   if (slices > 64) slices = 64;
   if ((int64_t)slices > (n + 63) / 64) slices = (int)((n + 63) / 64);
