@@ -291,6 +291,17 @@ __device__ __forceinline__ bool cand_less(double ka, uint32_t ia, double kb, uin
   return ka < kb || (!(kb < ka) && (ia & kIdMask) < (ib & kIdMask));
 }
 
+// cp.async of 16 aligned bytes (src_bytes 0: zeros), its groups and their waits.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 template <int KPL, typename K = float>
 struct WarpList {
   K key[KPL];

@@ -55,16 +55,6 @@ __device__ __forceinline__ bool hash_insert(int32_t* H, int hbits, int32_t id) {
   return false;  // unreachable: the table holds twice the most insertions
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
 }  // namespace
