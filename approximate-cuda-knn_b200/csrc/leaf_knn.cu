@@ -112,10 +112,6 @@ __device__ __forceinline__ int warp_dim_list(MaskFn word, int W, int d, int dpad
 
 // Dim lists are 16-bit (dims below 32768), in global memory (a leaf block's
 // list) or shared memory (a tile pair's): generic loads serve both.
-__device__ __forceinline__ int4 load_dims4(const int16_t* p) {
-  const short4 v = *reinterpret_cast<const short4*>(p);
-  return make_int4(v.x, v.y, v.z, v.w);
-}
 __device__ __forceinline__ int load_dim(const int16_t* p) { return *p; }
 
 // One warp per leaf: the listed dims of every 256-dim group in increasing order,
@@ -279,6 +275,15 @@ __global__ void __launch_bounds__(256) k_tile_dim_mask(const float* __restrict__
 // (all dims, or the listed non-zero dims dl of a sparse block) in the
 // reference's order: a sequential partial per 256-dim group, added to the
 // total at the group's end.  Ks receives the keys, +inf outside mq x mc.
+//
+// Listed dims: a lane per dim of the chunk, so that a warp's load covers one row's
+// few lines (a lane per row and four listed dims touched twenty), and the padded dims
+// past the chunk's last are skipped eight at a time (exact zeros).  Stores go down a
+// column of Qs: the pitch moves a dim by four banks, and with 64-row tiles, read
+// four rows at a time, the rows of four turn by one per eight dims, so that a warp's
+// 32 dims fall into 32 banks.
+// B200, 250,000 x 784 L1, leaves of 31,250, four trees: 615 -> 534 ms in this kernel with
+// merge_rows's SKIP; the next chunk fetched by 4-byte cp.async meanwhile: 582.
 template <int METRIC, int TILE>
 __device__ __forceinline__ void tile_keys(const float* __restrict__ X, int dpad, const int16_t* dl,
                                           int nchunks, int mq, int mc, const int32_t* qid, const int32_t* cid,
@@ -294,53 +299,65 @@ __device__ __forceinline__ void tile_keys(const float* __restrict__ X, int dpad,
       part[a][b] = 0.f;
       total[a][b] = 0.f;
     }
+  // where row r of dim e is kept, and which row of four position v holds
+  auto turned = [](int e, int r) { return R == 4 ? (r & ~3) | ((r + (e >> 3)) & 3) : r; };
   for (int ch = 0; ch < nchunks; ++ch) {
     const int cd = ch * kDC;
+    int lim = kDC;
+    if (dl) {
+      const int warp = tid >> 5, lane = tid & 31;
+      const int dim = load_dim(dl + cd + lane);  // -1: padding, kept as zero
+      lim = __popc(__ballot_sync(0xFFFFFFFFu, dim >= 0));
+      constexpr int RW = TILE / 8;
 #pragma unroll
-    for (int h = 0; h < TILE / 32; ++h) {
-      const int f = tid + h * 256;
-      const int r = f >> 3, c4 = f & 7;
-      float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), cv = qv;
-      if (dl) {  // four listed dims (-1: padding, read as zero)
-        const int4 dm = load_dims4(dl + cd + 4 * c4);
-        if (r < mq) {
-          const float* row = X + (size_t)qid[r] * dpad;
-          if (dm.x >= 0) qv.x = __ldg(row + dm.x);
-          if (dm.y >= 0) qv.y = __ldg(row + dm.y);
-          if (dm.z >= 0) qv.z = __ldg(row + dm.z);
-          if (dm.w >= 0) qv.w = __ldg(row + dm.w);
+      for (int side = 0; side < 2; ++side) {
+        const int32_t* id = side ? cid : qid;
+        const int m = side ? mc : mq;
+        float v[RW];
+#pragma unroll
+        for (int u = 0; u < RW; ++u) {
+          const int r = warp * RW + u;
+          v[u] = dim >= 0 && r < m ? __ldg(X + (size_t)id[r] * dpad + dim) : 0.f;
         }
-        if (r < mc) {
-          const float* row = X + (size_t)cid[r] * dpad;
-          if (dm.x >= 0) cv.x = __ldg(row + dm.x);
-          if (dm.y >= 0) cv.y = __ldg(row + dm.y);
-          if (dm.z >= 0) cv.z = __ldg(row + dm.z);
-          if (dm.w >= 0) cv.w = __ldg(row + dm.w);
-        }
-      } else {
+#pragma unroll
+        for (int u = 0; u < RW; ++u) (side ? Cs : Qs)[lane][turned(lane, warp * RW + u)] = v[u];
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < TILE / 32; ++h) {
+        const int f = tid + h * 256;
+        const int r = f >> 3, c4 = f & 7;
+        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), cv = qv;
         const int dim = cd + 4 * c4;
         if (r < mq && dim < dpad) qv = __ldg(reinterpret_cast<const float4*>(X + (size_t)qid[r] * dpad + dim));
         if (r < mc && dim < dpad) cv = __ldg(reinterpret_cast<const float4*>(X + (size_t)cid[r] * dpad + dim));
+        const int rt = turned(4 * c4, r);  // the same for the four dims
+        Qs[4 * c4 + 0][rt] = qv.x;
+        Qs[4 * c4 + 1][rt] = qv.y;
+        Qs[4 * c4 + 2][rt] = qv.z;
+        Qs[4 * c4 + 3][rt] = qv.w;
+        Cs[4 * c4 + 0][rt] = cv.x;
+        Cs[4 * c4 + 1][rt] = cv.y;
+        Cs[4 * c4 + 2][rt] = cv.z;
+        Cs[4 * c4 + 3][rt] = cv.w;
       }
-      Qs[4 * c4 + 0][r] = qv.x;
-      Qs[4 * c4 + 1][r] = qv.y;
-      Qs[4 * c4 + 2][r] = qv.z;
-      Qs[4 * c4 + 3][r] = qv.w;
-      Cs[4 * c4 + 0][r] = cv.x;
-      Cs[4 * c4 + 1][r] = cv.y;
-      Cs[4 * c4 + 2][r] = cv.z;
-      Cs[4 * c4 + 3][r] = cv.w;
     }
     __syncthreads();
-#pragma unroll 8
-    for (int dd = 0; dd < kDC; ++dd) {
-      float qa[R], cb[R];
-      load_r<R>(&Qs[dd][ty * R], qa);
-      load_r<R>(&Cs[dd][tx * R], cb);
 #pragma unroll
-      for (int a = 0; a < R; ++a)
+    for (int s = 0; s < kDC / 8; ++s) {
+      if (8 * s >= lim) break;  // block-uniform
 #pragma unroll
-        for (int b = 0; b < R; ++b) part[a][b] = acc_step<METRIC>(qa[a], cb[b], part[a][b]);
+      for (int dd = 8 * s; dd < 8 * s + 8; ++dd) {
+        float qa[R], cb[R];
+        load_r<R>(&Qs[dd][ty * R], qa);
+        load_r<R>(&Cs[dd][tx * R], cb);
+        const int turn = R == 4 ? s : 0;
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+#pragma unroll
+          for (int b = 0; b < R; ++b)
+            part[a][b] = acc_step<METRIC>(qa[(a + turn) & (R - 1)], cb[(b + turn) & (R - 1)], part[a][b]);
+      }
     }
     // end of a 256-dim group: its partial sum joins the total
     const bool gend = ch == nchunks - 1 ||
@@ -445,15 +462,27 @@ __device__ __forceinline__ bool pair_out(const float* __restrict__ X, int dpad, 
 // Merge rows rowid[0..mrow) of a tile into their running sorted lists against
 // the tile's columns colid[0..mcol): keys Ks[row][col], or Ks[col][row] when
 // TRANS (the tile read from its other side: every key is symmetric in its two
-// points, bit for bit).  One warp per row: bitonic insertion via shuffles.
-template <int KPL, int TILE, bool TRANS>
+// points, bit for bit).  One warp per row: bitonic insertion via shuffles.  SKIP: rows
+// whose last key is below all of the tile's are passed over without reading their
+// lists.  In leaves of many tiles (pairs) that is most rows once the lists have filled;
+// the small leaves of k_leaf enter nearly every row's list, and the test cost 6 % there.
+template <int KPL, int TILE, bool TRANS, bool SKIP>
 __device__ __forceinline__ void merge_rows(int k, int mrow, int mcol, const int32_t* rowid, const int32_t* colid,
                                            const float (*Ks)[TILE + 1], float* __restrict__ rkey,
                                            uint32_t* __restrict__ rid) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float kInf = __int_as_float(0x7F800000);
+  const int own = warp + 8 * lane;
+  const float tails = SKIP && own < mrow ? rkey[(size_t)rowid[own] * k + k - 1] : 0.f;
   for (int rr = warp; rr < mrow; rr += 8) {
     const uint32_t i = (uint32_t)rowid[rr];
+    if (SKIP) {
+      const float last = __shfl_sync(0xFFFFFFFFu, tails, rr >> 3);
+      bool any = false;
+#pragma unroll
+      for (int c = lane; c < TILE; c += 32) any |= c < mcol && !((TRANS ? Ks[c][rr] : Ks[rr][c]) > last);
+      if (!__any_sync(0xFFFFFFFFu, any)) continue;
+    }
     WarpList<KPL> L;
 #pragma unroll
     for (int r = 0; r < KPL; ++r) {
@@ -561,7 +590,7 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf(const float* _
       __syncthreads();
       tile_keys<METRIC, TILE>(X, dpad, dl, nchunks, mq, mc, qid, cid, qnorm, cnorm, Qs, Cs, Ks);
       __syncthreads();
-      merge_rows<KPL, TILE, false>(k, mq, mc, qid, cid, Ks, rkey, rid);
+      merge_rows<KPL, TILE, false, false>(k, mq, mc, qid, cid, Ks, rkey, rid);
       __syncthreads();
     }
   }
@@ -660,8 +689,8 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf_pair(
     return;
   tile_keys<METRIC, TILE>(X, dpad, dl, nchunks, mq, mc, qid, cid, qnorm, cnorm, Qs, Cs, Ks);
   __syncthreads();
-  merge_rows<KPL, TILE, false>(k, mq, mc, qid, cid, Ks, rkey, rid);
-  if (a != b) merge_rows<KPL, TILE, true>(k, mc, mq, cid, qid, Ks, rkey, rid);
+  merge_rows<KPL, TILE, false, true>(k, mq, mc, qid, cid, Ks, rkey, rid);
+  if (a != b) merge_rows<KPL, TILE, true, true>(k, mc, mq, cid, qid, Ks, rkey, rid);
 }
 
 // Rounds of the pair schedule for leaves of at most maxleaf points: T' = the
