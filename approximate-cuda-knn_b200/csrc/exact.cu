@@ -484,6 +484,14 @@ __global__ void k_exact_merge(int64_t nq, int k, int slices, const double* __res
   }
 }
 
+// A slice starts with open lists, whose pairs all get FP64 keys: the filter pays where
+// the slice is long against that and k (1088 queries x 25,787 x 14, k=28, slices of
+// 759: 2.32 -> 2.11 ms).  Past k = 32 the lists' registers leave one block per SM
+// (1721 x 28,652 x 169, k=33, slices of 1365: 7.44 -> 7.03 ms, and slower below).
+bool exact_filter_applies(int64_t slice, int k, int d) {
+  return slice >= 512 + (k <= 32 ? 8 : 32) * (int64_t)k && d <= kFilterMaxDim;
+}
+
 int exact_fp64(const float* X, int64_t n, int d, int dpad, int k, int metric,
                const int64_t* queries, int64_t nq, double* norms, double* part_dist,
                uint32_t* part_idx, int slices, double* out_dist, int32_t* out_idx,
@@ -493,15 +501,13 @@ int exact_fp64(const float* X, int64_t n, int d, int dpad, int k, int metric,
   const int64_t slice = (n + slices - 1) / slices;
   dim3 grid((unsigned)((nq + kET - 1) / kET), (unsigned)slices);
   const int kpl = kpl_for(k);
-  // A slice starts with open lists, whose pairs all get FP64 keys: the filter pays where
-  // the slice is long against that and k (500 queries x 50,000 x 64, k=16, slices of 782:
-  // 2.28 -> 1.92 ms; shorter slices go to k_exact alone, as before).
-  const bool filter = slice >= 512 + 8 * k && d <= kFilterMaxDim;
+  const bool filter = exact_filter_applies(slice, k, d);
   const bool vec = (dpad & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
 #define KNN_EXACT(M, KP)                                                                                            \
   do {                                                                                                              \
+    /* also where the filter stays off: it loads the kernel, so that a warm-up call does */                          \
+    cudaFuncSetAttribute(k_exact_filtered<M, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FilterSmem)); \
     if (filter) {                                                                                                   \
-      cudaFuncSetAttribute(k_exact_filtered<M, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FilterSmem)); \
       k_exact_filtered<M, KP><<<grid, 256, sizeof(FilterSmem), st>>>(X, n, d, dpad, vec, k, queries, nq, norms, slice, \
                                                                      part_dist, part_idx);                          \
     }                                                                                                               \

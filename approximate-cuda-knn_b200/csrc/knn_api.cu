@@ -20,6 +20,7 @@
 #include "knn_kernels.cuh"
 
 namespace knn {
+bool exact_filter_applies(int64_t slice, int k, int d);
 int exact_fp64(const float* X, int64_t n, int d, int dpad, int k, int metric,
                const int64_t* queries, int64_t nq, double* norms, double* part_dist,
                uint32_t* part_idx, int slices, double* out_dist, int32_t* out_idx,
@@ -1778,8 +1779,10 @@ int knn_exact_fp64(knn_context* ctx, const void* points, int64_t n, int32_t d, i
   int dev_sms = 148;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int64_t qtiles = (nq + 63) / 64;
-  // two whole waves of two blocks per SM, never a third wave of a few blocks
-  int slices = (int)((4LL * dev_sms) / qtiles);
+  int slices = (int)((4LL * dev_sms + qtiles - 1) / qtiles);
+  // the filter runs two blocks per SM: two whole waves, not a third of a few blocks
+  const int64_t whole = std::min<int64_t>(64, std::max<int64_t>(1, 4LL * dev_sms / qtiles));
+  if (knn::exact_filter_applies((n + whole - 1) / whole, k, d)) slices = (int)whole;
   if (slices < 1) slices = 1;
   if (slices > 64) slices = 64;
   if ((int64_t)slices > (n + 63) / 64) slices = (int)((n + 63) / 64);

@@ -23,7 +23,7 @@ def _check(oracle, x, k, metric, nq, seed=0):
 # 1700 queries: 27 query tiles, 21 slices, so these n give slices past the filter's shortest
 @pytest.mark.parametrize("metric", [0, 1, 2])
 @pytest.mark.parametrize("d,k,n", [(1, 5, 13001), (4, 8, 14000), (15, 16, 15013), (16, 10, 15013), (17, 30, 17000),
-                                   (37, 33, 19000), (64, 64, 24001), (130, 100, 31007)])
+                                   (37, 33, 34000), (64, 64, 55001), (130, 100, 79007)])
 def test_shapes(oracle, metric, d, k, n):
     acknn = load_package()
     _check(oracle, acknn.workloads.gaussian_mixture(n, d, 8, seed=d), k, metric, 1700, d)
@@ -49,3 +49,23 @@ def test_range(oracle, metric, scale):
     x = (x / np.abs(x).max() * 3.0 * scale).astype(np.float32)
     x[::3] *= np.float32(1e-3)
     _check(oracle, x, 12, metric, 1700)
+
+
+@pytest.mark.parametrize("metric", [0, 1, 2])
+@pytest.mark.parametrize("d", [7, 18])
+def test_rows_in_place(oracle, metric, d):
+    """The entry point without allocation reads the caller's rows, here off 16-byte boundaries."""
+    torch = pytest.importorskip("torch")
+    acknn = load_package()
+    lib = acknn.load_library()
+    n, k, nq = 15000, 10, 1700
+    x = acknn.workloads.gaussian_mixture(n, d, 8, seed=d)
+    q = np.arange(3, 3 + nq, dtype=np.int64)
+    xd, qd = torch.from_numpy(x).cuda(), torch.from_numpy(q).cuda()
+    idx = torch.empty((nq, k), dtype=torch.int32, device="cuda")
+    dist = torch.empty((nq, k), dtype=torch.float64, device="cuda")
+    assert lib.knn_exact_fp64_noalloc(xd.data_ptr(), n, d, k, metric, qd.data_ptr(), nq, idx.data_ptr(),
+                                      dist.data_ptr(), None) == 0
+    oi, od = oracle.exact(x, k, q, metric)
+    np.testing.assert_array_equal(idx.cpu().numpy(), oi)
+    np.testing.assert_array_equal(dist.cpu().numpy().view(np.uint64), od.view(np.uint64))
