@@ -262,6 +262,7 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 // Lists and candidates are (ordered key, id) pairs compared as one 64-bit
 // number: ordered keys are the FP32 keys mapped to integers of the same order.
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+constexpr uint32_t kInfKey = 0xFF800000u;  // +inf
 __device__ __forceinline__ float from_orderable(uint32_t o) {
   return __uint_as_float((o & 0x80000000u) ? (o ^ 0x80000000u) : ~o);
 }
@@ -506,8 +507,11 @@ __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, 
           }
           const float dot = __uint_as_float(v.x);
           const uint32_t p = v.y;
-          ck[i] = orderable(METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(xn, np[p]))
-                                                           : __fsub_rn(1.f, dot));
+          // a key that is not a number (rows with infinite values) goes last: its sign bit, which
+          // would rank it, depends on how the expression was compiled
+          const float key = METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(xn, np[p]))
+                                                           : __fsub_rn(1.f, dot);
+          ck[i] = key < __int_as_float(0x7F800000) ? orderable(key) : kInfKey;
           ci[i] = (uint32_t)perm[p];
         }
       }
