@@ -83,10 +83,14 @@ struct knn_context {
   // the tensor-core tile kernels of that build to stop issuing work; [1] is
   // sticky -- set with [0] by a kernel whose bounded wait gave up, and cleared
   // only when a synchronising call or knn_context_status() reports it, so an
-  // asynchronous build's failure reaches the caller.
+  // asynchronous build's failure reaches the caller.  [2] and [3] take the same
+  // writes from the FP32 leaf filter, whose give-ups are no failure (dense tiles
+  // take the tree), and are not read.
   int* err_words = nullptr;
-  // Test hook: the next build starts with both error words set.
+  // Test hook: the next build starts as if its tile waits had given up (tensor-core
+  // precisions: both error words set; FP32: the leaf filter's blocks).
   bool preset_err = false;
+  bool filter_gives_up = false;  // this build's
   // Events around each tree's leaf-tile kernel (statistics only), grown on demand.
   std::vector<cudaEvent_t> kev;
   cudaEvent_t* kernel_events(int trees) {
@@ -167,8 +171,8 @@ int make_context(int device, knn_context** out) {
   KNN_CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   for (auto& ev : c->ev) KNN_CK(cudaEventCreate(&ev));
   for (auto& ev : c->tev) KNN_CK(cudaEventCreate(&ev));
-  KNN_CK(cudaMalloc(&c->err_words, 2 * sizeof(int)));
-  KNN_CK(cudaMemset(c->err_words, 0, 2 * sizeof(int)));
+  KNN_CK(cudaMalloc(&c->err_words, 4 * sizeof(int)));
+  KNN_CK(cudaMemset(c->err_words, 0, 4 * sizeof(int)));
   *out = c.release();
   return KNN_OK;
 }
@@ -532,7 +536,8 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
   f.rkey = a.rkey;
   f.rid = a.rid;
   f.pair_counter = counter;
-  f.err = C->err_words;
+  f.err = C->err_words + 2;
+  f.give_up = C->filter_gives_up;
   f.kev = kev;
   f.stream = st;
   rc = C->get("Xp", (size_t)n * knn::umma_row_stride(d) * 2, &f.Xp);
@@ -1006,11 +1011,13 @@ int enter_device(knn_context** ctx, const knn_options& o) {
   return KNN_OK;
 }
 
-// Start of a build: clear the per-build error word (or set both words for the
-// test hook) on the build's stream.
-int reset_error_word(knn_context* C, cudaStream_t st) {
-  if (C->preset_err) {
-    C->preset_err = false;
+// Start of a build: clear the per-build error word (or act on the test hook) on
+// the build's stream.
+int reset_error_word(knn_context* C, int precision, cudaStream_t st) {
+  const bool preset = C->preset_err;
+  C->preset_err = false;
+  C->filter_gives_up = preset && precision == KNN_PREC_FP32;
+  if (preset && precision != KNN_PREC_FP32) {
     KNN_CK(cudaMemsetAsync(C->err_words, 0x01, 2 * sizeof(int), st));
   } else {
     KNN_CK(cudaMemsetAsync(C->err_words, 0, sizeof(int), st));
@@ -1087,7 +1094,7 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
   rc = get_lists(C, n, k, &L);
   if (rc) return rc;
   int* err_flag = C->err_words;
-  rc = reset_error_word(C, st);
+  rc = reset_error_word(C, o.precision, st);
   if (rc) return rc;
   const bool tensor_leaf = o.precision != KNN_PREC_FP32 && metric != KNN_METRIC_TAXICAB &&
                            d <= 256 && k <= 32;
@@ -1368,11 +1375,11 @@ int batch_impl(knn_context* C, const knn_dataset* sets, int count, int32_t k, in
   for (int i = 0; i < count; ++i) by_d[sets[i].d].push_back(i);
   int max_depth = 0;
   int* err_flag = C->err_words;
-  int rc = reset_error_word(C, st);
+  int rc = reset_error_word(C, o.precision, st);
   if (rc) return rc;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   KNN_CK(cudaStreamIsCapturing(st, &cs));
-  if (cs != cudaStreamCaptureStatusNone || timed) use_graphs = false;
+  if (cs != cudaStreamCaptureStatusNone || timed || C->filter_gives_up) use_graphs = false;
   float stage_ms[3] = {0, 0, 0};
 
   for (auto& kv : by_d) {

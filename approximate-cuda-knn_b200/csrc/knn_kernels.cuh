@@ -196,7 +196,8 @@ struct FilterLeafArgs {
   // launches tree t's dense tiles, which run if *survivors > limit
   std::function<int(int t, const unsigned long long* survivors, unsigned long long limit)> dense_tree;
   unsigned long long* pair_counter;
-  int* err;
+  int* err;                 // [2], written when a wait gives up, which only hands the tree to dense tiles
+  bool give_up;             // test hook: as if every wait gave up
   cudaEvent_t* kev;
   cudaStream_t stream;
 };

@@ -148,6 +148,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // (globaltimer) have passed, or once another wait of the block has given up.
 // The first to give up records it in the block's status and the error words:
 // err[0] stops the build's later blocks, err[1] stays until the host reports it.
+// (FP32 filter: words that nobody reads; the block hands its tree to dense tiles.)
 constexpr uint64_t kWaitNs = 20ull * 1000 * 1000;  // 20 ms; a tile takes under a microsecond
 constexpr uint32_t kSpinLimit = 1u << 20;
 __device__ __forceinline__ uint64_t global_ns() {
@@ -162,6 +163,8 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volat
     if (*status != 0) return false;
     if (global_ns() - t0 > kWaitNs) break;
   }
+  // the time may have passed between the last poll and the clock (a time-sliced GPU)
+  if (mbar_try_wait(bar, parity)) return true;
   *status = 1;
   atomicExch(err, 1);
   atomicOr(err + 1, 1);
@@ -377,6 +380,7 @@ struct LeafTcArgs {
   unsigned long long* pair_counter;
   unsigned long long* survivors;  // FP32 filter: [-1] of the tree before, [0] of this tree
   unsigned long long survivor_limit;
+  bool give_up;           // test hook: every block behaves as if a wait had given up
   float g, g1;            // FP32 rounding of a key; of a tile's sums
   int d, dpad, metric;
   uint32_t* count;        // [blocks of the launch][128 QT] survivors of each row, kListed
@@ -613,8 +617,9 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
       }
       mbar_init(bar_done, 1);
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-      // an earlier block of the build gave up (or dense tiles take the tree): do nothing
-      *status_p = *reinterpret_cast<volatile int*>(a.err) != 0 || (BOUND && too_many(a, -1)) ? 2 : 0;
+      // an earlier block of the build gave up: do nothing.  FP32 filter: dense tiles take the tree
+      if (BOUND) *status_p = too_many(a, -1) || too_many(a, 0) ? 2 : a.give_up ? 1 : 0;
+      else *status_p = *reinterpret_cast<volatile int*>(a.err) != 0 ? 2 : 0;
     }
     __syncwarp();
   } else if (warp == 4 * QT + 1) {  // MMA warp: tensor memory
@@ -1040,6 +1045,8 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
+  // FP32 filter: a block whose wait gave up leaves its tree to the dense tiles
+  if (BOUND && tid == 0 && *status == 1) atomicMax(a.survivors, a.survivor_limit + 1ull);
   if (warp == 4 * QT + 1) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)Plan::kTotal));
@@ -1089,7 +1096,6 @@ __global__ void __launch_bounds__(kBM * QT, 10 / QT) k_leaf_tc_exact(const __gri
   unsigned char* slice = slices + (threadIdx.x >> 5) * kExactBytes;
   const int row = range.q0 + (int)threadIdx.x;
   const bool live = row < (int)(range.hi - range.lo) && lane * (int)gridDim.y >> 5 == (int)blockIdx.y;
-  if (*reinterpret_cast<volatile int*>(a.err) != 0) return;  // the build gave up: counts may be missing
   const float kInf = __int_as_float(0x7F800000);
   const size_t slot = (size_t)blockIdx.x * (kBM * QT) + threadIdx.x;
   const int64_t pos = range.lo + row;
@@ -1109,7 +1115,9 @@ __global__ void __launch_bounds__(kBM * QT, 10 / QT) k_leaf_tc_exact(const __gri
     const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)size);
     if (lane == 0 && sum) atomicAdd(a.pair_counter, (unsigned long long)sum);
   }
-  if (too_many(a, 0)) return;  // dense tiles follow (a later chunk's count may still decide so: they repeat this one)
+  // dense tiles follow (a later chunk's count may still decide so: they repeat this one), whether for the
+  // number of survivors or because a block gave up and left no counts
+  if (too_many(a, 0)) return;
   const uint32_t c = live ? a.count[slot] : 0u;
   if (!__any_sync(0xFFFFFFFFu, c != 0u)) return;
   const int qid = live ? a.perm[pos] : -1;
@@ -1694,6 +1702,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   t.rkey = a.rkey;
   t.maxabs = a.maxabs;
   t.pair_counter = a.pair_counter;
+  t.give_up = a.give_up;
   t.g = (float)(2 * a.d + 64) * 5.9604644775390625e-08f;   // 2^-24
   t.g1 = (float)(a.d + 64) * 4.76837158203125e-07f;        // 2^-21: the tensor cores' sums are not rounded to nearest
   t.d = a.d;

@@ -53,7 +53,11 @@ extern "C" {
 #define KNN_BF16 2
 
 /* Precision modes of the leaf stage. */
-#define KNN_PREC_FP32 0        /* every key in FP32 CUDA-core arithmetic          */
+#define KNN_PREC_FP32 0        /* every key in FP32 CUDA-core arithmetic; tensor-core
+                                  tiles may rule pairs out beforehand by bounds that
+                                  hold for the FP32 keys, and give up to dense FP32
+                                  tiles: the graph is the same, and a tile wait
+                                  is never a failure                             */
 #define KNN_PREC_BF16_RERANK 1 /* leaf blocks as BF16 tensor-core tiles in the
                                   |x|^2+|y|^2-2x.y form, each point's best 2k
                                   re-ranked with exact FP32 keys.  TAXICAB, and
@@ -184,9 +188,10 @@ int64_t knn_context_scratch_bytes(const knn_context* ctx);
 int knn_context_status(knn_context* ctx, void* stream);
 
 /* Test hook: the next build on `ctx` (NULL: the thread's default context)
- * starts with its tile-wait error word already set, as if a wait had given
- * up.  Its tensor-core tile kernels then issue no MMA, free their tensor
- * memory and return, and the build returns KNN_ERR_TIMEOUT.  One-shot; the
+ * starts as if a tile wait had given up.  Its tensor-core tile kernels then
+ * issue no MMA, free their tensor memory and return.  With a tensor-core
+ * precision the build returns KNN_ERR_TIMEOUT; a plain FP32 build, whose tiles
+ * are only a filter, takes dense FP32 tiles instead and succeeds.  One-shot; the
  * build after it runs normally. */
 int knn_test_fail_next_tile_wait(knn_context* ctx);
 
