@@ -1356,11 +1356,14 @@ int group_compute(knn_context* C, const BatchGroup& g, int k, int trees, int pro
   return KNN_OK;
 }
 
+// Everything that decides what group_compute launches.
 std::string group_signature(const BatchGroup& g, int k, int trees, int leaf, int props, int metric,
-                            int precision) {
-  std::string s = "d" + std::to_string(g.d) + ":k" + std::to_string(k) + ":t" + std::to_string(trees) + ":l" +
-                  std::to_string(leaf) + ":p" + std::to_string(props) + ":m" + std::to_string(metric) + ":q" +
-                  std::to_string(precision);
+                            const knn_options& o) {
+  std::string s = "d" + std::to_string(g.d);
+  for (const auto& f : {std::make_pair(":k", k), {":t", trees}, {":l", leaf}, {":p", props}, {":m", metric},
+                        {":q", o.precision}, {":T", o.leaf_tile}, {":S", o.sparse_dims}, {":P", o.tile_pairs},
+                        {":G", o.tc_group}, {":w", o.prop_warps}, {":a", o.autotune}})
+    s += f.first + std::to_string(f.second);
   for (const auto& e : g.hsegs) s += ":" + std::to_string(e.n) + "/" + std::to_string(e.seed);
   return s;
 }
@@ -1421,7 +1424,7 @@ int batch_impl(knn_context* C, const knn_dataset* sets, int count, int32_t k, in
     KNN_CK(cudaMemcpyAsync(dsegs, g.hsegs.data(), sizeof(knn::SegEntry) * nseg, cudaMemcpyHostToDevice, st));
     // compute: replay a captured graph of this shape, capture it on its second
     // sighting, or launch directly
-    const std::string sig = use_graphs ? group_signature(g, k, trees, leaf, props, metric, o.precision) : "";
+    const std::string sig = use_graphs ? group_signature(g, k, trees, leaf, props, metric, o) : "";
     bool done = false;
     if (use_graphs) {
       for (auto& cg : C->graphs)
