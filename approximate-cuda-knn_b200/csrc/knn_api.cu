@@ -83,9 +83,8 @@ struct knn_context {
   // the tensor-core tile kernels of that build to stop issuing work; [1] is
   // sticky -- set with [0] by a kernel whose bounded wait gave up, and cleared
   // only when a synchronising call or knn_context_status() reports it, so an
-  // asynchronous build's failure reaches the caller.  [2] and [3] take the same
-  // writes from the FP32 leaf filter, whose give-ups are no failure (dense tiles
-  // take the tree), and are not read.
+  // asynchronous build's failure reaches the caller.  (The FP32 leaf filter has
+  // words of its own: dense tiles take a tree whose waits give up.)
   int* err_words = nullptr;
   // Test hook: the next build starts as if its tile waits had given up (tensor-core
   // precisions: both error words set; FP32: the leaf filter's blocks).
@@ -171,8 +170,8 @@ int make_context(int device, knn_context** out) {
   KNN_CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   for (auto& ev : c->ev) KNN_CK(cudaEventCreate(&ev));
   for (auto& ev : c->tev) KNN_CK(cudaEventCreate(&ev));
-  KNN_CK(cudaMalloc(&c->err_words, 4 * sizeof(int)));
-  KNN_CK(cudaMemset(c->err_words, 0, 4 * sizeof(int)));
+  KNN_CK(cudaMalloc(&c->err_words, 2 * sizeof(int)));
+  KNN_CK(cudaMemset(c->err_words, 0, 2 * sizeof(int)));
   *out = c.release();
   return KNN_OK;
 }
@@ -536,7 +535,6 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
   f.rkey = a.rkey;
   f.rid = a.rid;
   f.pair_counter = counter;
-  f.err = C->err_words + 2;
   f.give_up = C->filter_gives_up;
   f.kev = kev;
   f.stream = st;
@@ -548,20 +546,15 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
   if (!rc) rc = C->get("survivors", srows * knn::umma_row_scratch_bytes(), &f.surv);
   if (!rc) rc = C->get("surv_count", srows, &f.count);
   if (!rc) rc = C->get("maxabs", 1, &f.maxabs);
-  if (!rc) rc = C->get("leaf_survivors", (size_t)trees + 1, &f.survivors);
+  if (!rc) rc = C->get("leaf_survivors", (size_t)trees + 2, &f.survivors);
   if (rc) return rc;
   f.dense_tree = [&](int t, const unsigned long long* survivors, unsigned long long limit) {
     knn::LeafArgs one = a;
     one.first_tree = t;
-    one.trees = 1;
-    one.pairs = false;
     one.guard = survivors;
     one.guard_limit = limit;
-    one.kev = nullptr;
     one.pair_counter = nullptr;  // the filter counts its pairs whichever way they are decided
-    one.dlist = nullptr;
-    one.tmask = nullptr;
-    return knn::leaf_stage(one, log);
+    return knn::leaf_stage_handed(one, log);
   };
   rc = knn::leaf_stage_filtered(f, log);
   if (rc) return fail_cuda(cudaGetLastError(), "filtered leaf stage launch");

@@ -106,7 +106,7 @@ struct LeafArgs {
   unsigned long long* pair_counter;  // optional
   int tile;              // 32 or 64 (0: 64): query x candidate tile, results identical
   int first_tree;        // trees [first_tree, first_tree + trees) of perm
-  const unsigned long long* guard;  // device word: one-sided tiles run only if it is above guard_limit (null: always)
+  const unsigned long long* guard;  // device word: the tiles run only if it is above guard_limit (leaf_stage: null)
   unsigned long long guard_limit;
   cudaEvent_t* kev;      // [2 * trees] events around each tree's tile kernel, or null
   const int64_t* ftable;
@@ -131,6 +131,9 @@ struct LeafArgs {
   cudaStream_t stream;
 };
 int leaf_stage(const LeafArgs& a, LaunchLog& log);
+// Tree first_tree alone, if *guard > guard_limit (EUCLIDEAN and COSINE, k <= 32, every leaf
+// its own block).
+int leaf_stage_handed(const LeafArgs& a, LaunchLog& log);
 
 // Mixed-precision leaf stage (BF16 tensor-core tiles + FP32 re-rank).
 struct UmmaLeafArgs {
@@ -192,11 +195,11 @@ struct FilterLeafArgs {
   void* surv;               // [filter_scratch_rows(...)][umma_row_scratch_bytes()] scratch
   uint32_t* count;          // [filter_scratch_rows(...)] scratch
   unsigned int* maxabs;
-  unsigned long long* survivors;  // [trees + 1] scratch: of each tree, after a zero
+  // [trees + 2] scratch: a zero, each tree's survivors, and the words of waits that gave up
+  unsigned long long* survivors;
   // launches tree t's dense tiles, which run if *survivors > limit
   std::function<int(int t, const unsigned long long* survivors, unsigned long long limit)> dense_tree;
   unsigned long long* pair_counter;
-  int* err;                 // [2], written when a wait gives up, which only hands the tree to dense tiles
   bool give_up;             // test hook: as if every wait gave up
   cudaEvent_t* kev;
   cudaStream_t stream;

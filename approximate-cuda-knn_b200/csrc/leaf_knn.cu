@@ -26,6 +26,7 @@ namespace knn {
 
 namespace {
 constexpr int kDC = 32;     // dims staged per chunk
+constexpr int kLocalInsertMax = 5;  // entrants up to which one-by-one insertion beats sort and merge
 }  // namespace
 
 // Register tile of R consecutive floats from shared memory (R = 2 or 4).
@@ -466,16 +467,19 @@ __device__ __forceinline__ bool pair_out(const float* __restrict__ X, int dpad, 
 // whose last key is below all of the tile's are passed over without reading their
 // lists.  In leaves of many tiles (pairs) that is most rows once the lists have filled;
 // the small leaves of k_leaf enter nearly every row's list, and the test cost 6 % there.
-template <int KPL, int TILE, bool TRANS, bool SKIP>
+// LOCAL: row rr's list is at rr * k (shared memory), not at its id's.
+template <int KPL, int TILE, bool TRANS, bool SKIP, bool LOCAL = false>
 __device__ __forceinline__ void merge_rows(int k, int mrow, int mcol, const int32_t* rowid, const int32_t* colid,
                                            const float (*Ks)[TILE + 1], float* __restrict__ rkey,
                                            uint32_t* __restrict__ rid) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float kInf = __int_as_float(0x7F800000);
   const int own = warp + 8 * lane;
-  const float tails = SKIP && own < mrow ? rkey[(size_t)rowid[own] * k + k - 1] : 0.f;
+  auto list = [&](int rr) { return (size_t)(LOCAL ? rr : rowid[rr]) * k; };
+  const float tails = SKIP && own < mrow ? rkey[list(own) + k - 1] : 0.f;
   for (int rr = warp; rr < mrow; rr += 8) {
     const uint32_t i = (uint32_t)rowid[rr];
+    const size_t at = list(rr);
     if (SKIP) {
       const float last = __shfl_sync(0xFFFFFFFFu, tails, rr >> 3);
       bool any = false;
@@ -488,8 +492,8 @@ __device__ __forceinline__ void merge_rows(int k, int mrow, int mcol, const int3
     for (int r = 0; r < KPL; ++r) {
       const int e = r * 32 + lane;
       if (e < k) {
-        L.key[r] = rkey[(size_t)i * k + e];
-        L.id[r] = rid[(size_t)i * k + e];
+        L.key[r] = rkey[at + e];
+        L.id[r] = rid[at + e];
       } else {
         L.key[r] = kInf;
         L.id[r] = kNoId;
@@ -507,15 +511,20 @@ __device__ __forceinline__ void merge_rows(int k, int mrow, int mcol, const int3
       if (!__any_sync(0xFFFFFFFFu, pass)) continue;
       const bool dup = warp_list_contains(L, ci, k);
       pass = pass && !dup;
-      if (!__any_sync(0xFFFFFFFFu, pass)) continue;
-      warp_list_insert(L, pass ? ck : kInf, pass ? ci : kNoId);
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, pass);
+      if (bal == 0) continue;
+      // few entrants: one by one (NaN keys, which have no order, as elsewhere)
+      if (LOCAL && __popc(bal) <= kLocalInsertMax && !__any_sync(0xFFFFFFFFu, (pass && ck != ck) || L.key[0] != L.key[0]))
+        warp_list_insert_lanes(L, bal, ck, ci, kInf);
+      else
+        warp_list_insert(L, pass ? ck : kInf, pass ? ci : kNoId);
     }
 #pragma unroll
     for (int r = 0; r < KPL; ++r) {
       const int e = r * 32 + lane;
       if (e < k) {
-        rkey[(size_t)i * k + e] = L.key[r];
-        rid[(size_t)i * k + e] = L.id[r];
+        rkey[at + e] = L.key[r];
+        rid[at + e] = L.id[r];
       }
     }
   }
@@ -532,9 +541,7 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf(const float* _
                                               float* __restrict__ rkey, uint32_t* __restrict__ rid,
                                               unsigned long long* __restrict__ pair_counter,
                                               const int16_t* __restrict__ dlist,
-                                              const int32_t* __restrict__ dnch, int lmax,
-                                              const unsigned long long* __restrict__ guard,
-                                              unsigned long long guard_limit) {
+                                              const int32_t* __restrict__ dnch, int lmax) {
   constexpr int kTile = TILE;
   static_assert(TILE == 32 || TILE == 64, "tile of 32 or 64");
   __shared__ __align__(16) float Qs[kDC][TILE + 4];
@@ -543,7 +550,6 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf(const float* _
   __shared__ int32_t qid[kTile], cid[kTile];
   __shared__ float qnorm[kTile], cnorm[kTile];
 
-  if (guard && *guard <= guard_limit) return;
   // block = (leaf, query tile): the 64-row (or 32-row) query tiles of a large
   // leaf spread over gridDim.y, and each query row's list is read and written
   // by one block only
@@ -593,6 +599,70 @@ __global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf(const float* _
       merge_rows<KPL, TILE, false, false>(k, mq, mc, qid, cid, Ks, rkey, rid);
       __syncthreads();
     }
+  }
+}
+
+// One tree's leaves, each its own block, that the tensor-core filter handed over (*guard
+// above the limit; else the grid returns at once).  One launch, as what decides is on the
+// device and every tree pays for the launches; the query rows' lists stay in shared
+// memory.  WHOLE: a block takes a leaf, each tile pair (a, b) once for both sides, in the
+// order a, b >= a; so a row meets the leaf's tiles in k_leaf's order, and lists with NaN
+// keys, which have no order, agree with it too.  Else one-sided tiles, a block per query tile.
+// What bounds it: keys and merges about evenly; see handed_whole for the figures.
+template <int METRIC, int TILE, bool WHOLE>
+__global__ void __launch_bounds__(256, TILE == 64 ? 4 : 5) k_leaf_handed(
+    const float* __restrict__ X, int d, int dpad, SegView segs, int64_t leaves, int k, const int32_t* __restrict__ perm,
+    const float* __restrict__ norms, float* __restrict__ rkey, uint32_t* __restrict__ rid,
+    const unsigned long long* __restrict__ guard, unsigned long long guard_limit, int rows, int tiles) {
+  __shared__ __align__(16) float Qs[kDC][TILE + 4];
+  __shared__ __align__(16) float Cs[kDC][TILE + 4];
+  __shared__ float Ks[TILE][TILE + 1];
+  __shared__ int32_t qid[TILE], cid[TILE];
+  __shared__ float qnorm[TILE], cnorm[TILE];
+  extern __shared__ __align__(16) unsigned char list_smem[];
+  float* lk = reinterpret_cast<float*>(list_smem);           // [rows][k]: the leaf's, or the query tile's
+  uint32_t* li = reinterpret_cast<uint32_t*>(lk + rows * k);  // [rows][k]
+  if (*guard <= guard_limit) return;
+  const int tid = threadIdx.x, nchunks = (d + kDC - 1) / kDC;
+  auto load_ids = [&](int64_t at, int m, int32_t* id, float* norm) {
+    if (tid < TILE) {
+      id[tid] = tid < m ? perm[at + tid] : -1;
+      if (METRIC == KNN_METRIC_COSINE) norm[tid] = tid < m ? norms[id[tid]] : 0.f;
+    }
+  };
+  for (int64_t item = blockIdx.x; item < leaves * tiles; item += gridDim.x) {
+    int64_t j;
+    const SegEntry seg = segs.leaf(item / tiles, &j);
+    const int64_t lo = seg.off + node_lo(seg.n, seg.depth, j);
+    const int n = (int)(seg.off + node_lo(seg.n, seg.depth, j + 1) - lo);
+    const int r0 = (int)(item % tiles) * TILE;  // first row (WHOLE: 0, one item a leaf)
+    if (r0 >= n) continue;                      // block-uniform
+    const int m = WHOLE ? n : min(TILE, n - r0);
+    for (int e = tid; e < m * k; e += 256) {
+      const size_t at = (size_t)perm[lo + r0 + e / k] * k + e % k;
+      lk[e] = rkey[at];
+      li[e] = rid[at];
+    }
+    for (int q0 = 0; q0 < m; q0 += TILE) {
+      const int mq = min(TILE, m - q0);
+      load_ids(lo + r0 + q0, mq, qid, qnorm);
+      for (int c0 = WHOLE ? q0 : 0; c0 < n; c0 += TILE) {
+        const int mc = min(TILE, n - c0);
+        load_ids(lo + c0, mc, cid, cnorm);
+        __syncthreads();
+        tile_keys<METRIC, TILE>(X, dpad, nullptr, nchunks, mq, mc, qid, cid, qnorm, cnorm, Qs, Cs, Ks);
+        __syncthreads();
+        merge_rows<1, TILE, false, true, true>(k, mq, mc, qid, cid, Ks, lk + q0 * k, li + q0 * k);
+        if (WHOLE && c0 != q0) merge_rows<1, TILE, true, true, true>(k, mc, mq, cid, qid, Ks, lk + c0 * k, li + c0 * k);
+        __syncthreads();
+      }
+    }
+    for (int e = tid; e < m * k; e += 256) {
+      const size_t at = (size_t)perm[lo + r0 + e / k] * k + e % k;
+      rkey[at] = lk[e];
+      rid[at] = li[e];
+    }
+    __syncthreads();  // the lists are replaced
   }
 }
 
@@ -749,14 +819,12 @@ static int launch_leaf_tile(const LeafArgs& a, const int32_t* perm, const int64_
   }
   const int64_t qtiles = (a.maxleaf + TILE - 1) / TILE;
   dim3 grid((unsigned)leaves, (unsigned)std::min<int64_t>(qtiles, 65535));
-  if (a.guard)  // most of these launches return at once: no more blocks than fill the chip
-    grid.y = (unsigned)std::min<int64_t>(grid.y, (8 * 148 + leaves - 1) / leaves);
   if (kpl == 1)
-    k_leaf<METRIC, 1, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax, a.guard, a.guard_limit);
+    k_leaf<METRIC, 1, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax);
   else if (kpl == 2)
-    k_leaf<METRIC, 2, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax, a.guard, a.guard_limit);
+    k_leaf<METRIC, 2, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax);
   else
-    k_leaf<METRIC, 4, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax, a.guard, a.guard_limit);
+    k_leaf<METRIC, 4, TILE><<<grid, 256, 0, a.stream>>>(a.X, a.d, a.dpad, a.segs, ftab, a.k, perm, a.norms, a.rkey, a.rid, a.pair_counter, dlist, a.dnch, a.lmax);
   return 1;
 }
 
@@ -799,6 +867,50 @@ int leaf_stage(const LeafArgs& a, LaunchLog& log) {
     else launch_leaf_metric<KNN_METRIC_COSINE>(a, t, kpl, log);
     if (a.kev) cudaEventRecord(a.kev[2 * (t - a.first_tree) + 1], a.stream);
   }
+  return cudaPeekAtLastError() == cudaSuccess ? KNN_OK : KNN_ERR_CUDA;
+}
+
+namespace {
+// Whole leaves where their lists leave room for three blocks per SM (EUCLIDEAN, whose keys take
+// two instructions per dim: for two) and there are two leaves per SM.  300,000 x 128, k = 16, six
+// trees all handed over, whole build in ms, EUCLIDEAN / COSINE (one infinite value):
+//   leaves of 293 (3 blocks):  whole 15.0 / 14.5, query tiles 16.3 / 14.3, k_leaf 22.1 / 20.3,
+//                              k_leaf_pair, a launch per round, 18.8 / 17.8
+//   leaves of 586 (2 blocks):  whole 24.7 / 26.7, query tiles 25.9 / 21.9, k_leaf 36.2 / 32.5,
+//                              k_leaf_pair 28.2 / 26.3
+// Clusters of 2 to 8 blocks per leaf, a barrier between the rounds of k_leaf_pair: 20.5 and 32.4.
+bool handed_whole(int metric, int64_t leaves, int64_t maxleaf, int k) {
+  return leaves >= 2 * 148 && maxleaf * k * 8 <= (metric == KNN_METRIC_EUCLIDEAN ? 76 : 39) * 1024;
+}
+
+template <int METRIC, int TILE, bool WHOLE>
+void launch_handed(const LeafArgs& a) {
+  const int rows = WHOLE ? (int)a.maxleaf : TILE;
+  const int64_t tiles = WHOLE ? 1 : (a.maxleaf + TILE - 1) / TILE;
+  const int smem = rows * a.k * 8;
+  cudaFuncSetAttribute(k_leaf_handed<METRIC, TILE, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // most of these launches return at once: no more blocks than fill the chip twice
+  const unsigned grid = (unsigned)std::min<int64_t>(a.leaves * tiles, 148 * 8);
+  k_leaf_handed<METRIC, TILE, WHOLE><<<grid, 256, smem, a.stream>>>(
+      a.X, a.d, a.dpad, a.segs, a.leaves, a.k, a.perm + (size_t)a.first_tree * a.n, a.norms, a.rkey, a.rid, a.guard,
+      a.guard_limit, rows, (int)tiles);
+}
+template <int METRIC, int TILE>
+void launch_handed_tile(const LeafArgs& a) {
+  if (handed_whole(METRIC, a.leaves, a.maxleaf, a.k)) launch_handed<METRIC, TILE, true>(a);
+  else launch_handed<METRIC, TILE, false>(a);
+}
+}  // namespace
+
+int leaf_stage_handed(const LeafArgs& a, LaunchLog& log) {
+  if (a.metric == KNN_METRIC_EUCLIDEAN) {
+    if (a.tile == 32) launch_handed_tile<KNN_METRIC_EUCLIDEAN, 32>(a);
+    else launch_handed_tile<KNN_METRIC_EUCLIDEAN, 64>(a);
+  } else {
+    if (a.tile == 32) launch_handed_tile<KNN_METRIC_COSINE, 32>(a);
+    else launch_handed_tile<KNN_METRIC_COSINE, 64>(a);
+  }
+  log.add();
   return cudaPeekAtLastError() == cudaSuccess ? KNN_OK : KNN_ERR_CUDA;
 }
 

@@ -148,7 +148,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // (globaltimer) have passed, or once another wait of the block has given up.
 // The first to give up records it in the block's status and the error words:
 // err[0] stops the build's later blocks, err[1] stays until the host reports it.
-// (FP32 filter: words that nobody reads; the block hands its tree to dense tiles.)
+// (FP32 filter: words of the build's own, no failure; the block hands its tree to dense tiles.)
 constexpr uint64_t kWaitNs = 20ull * 1000 * 1000;  // 20 ms; a tile takes under a microsecond
 constexpr uint32_t kSpinLimit = 1u << 20;
 __device__ __forceinline__ uint64_t global_ns() {
@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(64 + 128 * QT, TmemPlan<NCH, QT>::kBlocks)
       mbar_init(bar_done, 1);
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
       // an earlier block of the build gave up: do nothing.  FP32 filter: dense tiles take the tree
-      if (BOUND) *status_p = too_many(a, -1) || too_many(a, 0) ? 2 : a.give_up ? 1 : 0;
+      if (BOUND) *status_p = (int)too_many(a, -1) | (int)too_many(a, 0) ? 2 : a.give_up ? 1 : 0;
       else *status_p = *reinterpret_cast<volatile int*>(a.err) != 0 ? 2 : 0;
     }
     __syncwarp();
@@ -1096,6 +1096,7 @@ __global__ void __launch_bounds__(kBM * QT, 10 / QT) k_leaf_tc_exact(const __gri
   unsigned char* slice = slices + (threadIdx.x >> 5) * kExactBytes;
   const int row = range.q0 + (int)threadIdx.x;
   const bool live = row < (int)(range.hi - range.lo) && lane * (int)gridDim.y >> 5 == (int)blockIdx.y;
+  if (*reinterpret_cast<volatile int*>(a.err) != 0) return;  // a block gave up: dense tiles take the tree
   const float kInf = __int_as_float(0x7F800000);
   const size_t slot = (size_t)blockIdx.x * (kBM * QT) + threadIdx.x;
   const int64_t pos = range.lo + row;
@@ -1115,9 +1116,7 @@ __global__ void __launch_bounds__(kBM * QT, 10 / QT) k_leaf_tc_exact(const __gri
     const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)size);
     if (lane == 0 && sum) atomicAdd(a.pair_counter, (unsigned long long)sum);
   }
-  // dense tiles follow (a later chunk's count may still decide so: they repeat this one), whether for the
-  // number of survivors or because a block gave up and left no counts
-  if (too_many(a, 0)) return;
+  if (too_many(a, 0)) return;  // dense tiles follow (a later chunk's count may still decide so: they repeat this one)
   const uint32_t c = live ? a.count[slot] : 0u;
   if (!__any_sync(0xFFFFFFFFu, c != 0u)) return;
   const int qid = live ? a.perm[pos] : -1;
@@ -1687,7 +1686,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   t.dp = a.dp;
   t.segs = a.segs;
   t.aid = a.rid;
-  t.err = a.err;
+  t.err = reinterpret_cast<int*>(a.survivors + a.trees + 1);
   t.n = a.n;
   t.idesc = idesc_for(true);
   t.ldr = ldr;
@@ -1713,7 +1712,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   // would send most pairs down the survivors' path, at several times a dense
   // tile's cost (400,000 x 256, leaf 1,000, all pairs: 415 ms against 64), so from
   // an eighth of the pairs and 16 + k a row the dense tiles take over.
-  cudaMemsetAsync(a.survivors, 0, sizeof(unsigned long long) * (size_t)(a.trees + 1), st);
+  cudaMemsetAsync(a.survivors, 0, sizeof(unsigned long long) * (size_t)(a.trees + 2), st);
   t.survivor_limit = (unsigned long long)a.n * (unsigned long long)(16 + a.k + a.maxleaf / 8);
   for (int tr = a.first_tree; tr < a.trees; ++tr) {
     if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
