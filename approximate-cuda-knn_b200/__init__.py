@@ -150,6 +150,7 @@ EXPORTS = {
     "knn_context_scratch_bytes": (_I64, [_P]),
     "knn_context_status": (ctypes.c_int, [_P, _P]),
     "knn_test_fail_next_tile_wait": (ctypes.c_int, [_P]),
+    "knn_test_limit_scratch": (ctypes.c_int, [_P, _I64]),
     "knn_build": (ctypes.c_int, [_P, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _U64, _P, _P]),
     "knn_build_ex": (ctypes.c_int, [_P, _P, _I64, _I32, _I32, _I32, _I32, _I32, _I32, _U64, _P,
                                     _P, _P, _P]),

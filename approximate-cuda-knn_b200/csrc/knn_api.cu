@@ -50,6 +50,9 @@ int fail_cuda(cudaError_t e, const char* where) {
 struct Buffer {
   void* p = nullptr;
   size_t bytes = 0;
+  uint64_t used = 0;     // the call that last asked for it
+  size_t refused = 0;    // spare scratch: a size that there was no memory for,
+  uint64_t refused_at = 0;  // and the call that found out
 };
 
 }  // namespace
@@ -101,27 +104,59 @@ struct knn_context {
     return kev.data();
   }
 
+  // Number of the current call (each group of a batch counts as one).  Buffers that
+  // it has not asked for are given back when an allocation fails.
+  uint64_t call = 0;
+  int64_t scratch_limit = 0;  // test hook: bytes past which allocations fail (0: none)
+
+  cudaError_t allocate(void** p, size_t bytes) {
+    if (scratch_limit > 0 && bytes_held() + (int64_t)bytes > scratch_limit) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+  }
+  // cudaFree waits for the work that was queued before it.
+  cudaError_t give_back(Buffer& b) {
+    if (!b.p) return cudaSuccess;
+    const cudaError_t e = cudaFree(b.p);
+    b.p = nullptr;
+    b.bytes = 0;
+    ++generation;
+    return e;
+  }
   // Device buffer `name` of at least `bytes`; grows by reallocation.
-  int get(const char* name, size_t bytes, void** out) {
+  cudaError_t acquire(const char* name, size_t bytes, void** out) {
     Buffer& b = bufs[name];
     if (bytes == 0) bytes = 16;
+    b.used = call;
+    *out = nullptr;
     if (b.bytes < bytes) {
-      if (b.p) {
-        cudaError_t e = cudaFree(b.p);
-        b.p = nullptr;
-        b.bytes = 0;
-        if (e != cudaSuccess) return fail_cuda(e, "cudaFree");
+      cudaError_t e = give_back(b);
+      if (e != cudaSuccess) return e;
+      e = allocate(&b.p, bytes);
+      if (e == cudaErrorMemoryAllocation) {
+        bool any = false;
+        for (auto& kv : bufs)
+          if (kv.second.p && kv.second.used != call) {
+            e = give_back(kv.second);
+            if (e != cudaSuccess) return e;
+            any = true;
+          }
+        e = any ? allocate(&b.p, bytes) : cudaErrorMemoryAllocation;
       }
-      cudaError_t e = cudaMalloc(&b.p, bytes);
       if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail_cuda(e, (std::string("cudaMalloc ") + name).c_str());
+        b.p = nullptr;
+        return e;
       }
       b.bytes = bytes;
       ++generation;
     }
     *out = b.p;
-    return KNN_OK;
+    return cudaSuccess;
+  }
+  int get(const char* name, size_t bytes, void** out) {
+    const cudaError_t e = acquire(name, bytes, out);
+    return e == cudaSuccess ? KNN_OK : fail_cuda(e, (std::string("cudaMalloc ") + name).c_str());
   }
   template <typename T>
   int get(const char* name, size_t count, T** out) {
@@ -129,6 +164,39 @@ struct knn_context {
     int rc = get(name, count * sizeof(T), &p);
     *out = static_cast<T*>(p);
     return rc;
+  }
+  // Scratch that a call can do without: false where memory is short.  To be asked for
+  // after everything that the call needs.  A size that failed is tried again only some
+  // calls later, so that repeated calls do not free and allocate each time.
+  bool spare(const char* name, size_t bytes, void** out) {
+    constexpr uint64_t kRetryCalls = 16;
+    Buffer& b = bufs[name];
+    if (b.bytes < bytes && b.refused && bytes >= b.refused && call - b.refused_at < kRetryCalls) return false;
+    if (acquire(name, bytes, out) == cudaSuccess) return true;
+    b.refused = bytes;
+    b.refused_at = call;
+    return false;
+  }
+  template <typename T>
+  bool spare(const char* name, size_t count, T** out) {
+    void* p = nullptr;
+    const bool ok = spare(name, count * sizeof(T), &p);
+    *out = static_cast<T*>(p);
+    return ok;
+  }
+  // Survivor scratch of `rows` rows, or of as many halvings of that (at least `least`) as there
+  // is memory for: the rows that a launch of the leaf tiles may take, 0 if none.
+  size_t spare_survivors(size_t rows, size_t least, void** surv, uint32_t** count) {
+    for (; rows >= least; rows /= 2)
+      if (spare("survivors", rows * knn::umma_row_scratch_bytes(), surv) && spare("surv_count", rows, count)) return rows;
+    return 0;
+  }
+  // The named buffers are no longer in use by this call's later launches.
+  void done_with(std::initializer_list<const char*> names) {
+    for (const char* n : names) {
+      auto it = bufs.find(n);
+      if (it != bufs.end()) it->second.used = 0;
+    }
   }
   int64_t bytes_held() const {
     int64_t s = 0;
@@ -375,8 +443,9 @@ struct Lists {
 
 int get_lists(knn_context* C, int64_t n, int k, Lists* L) {
   const int kw = (k + 31) / 32;
-  int rc = C->get("key0", (size_t)n * k, &L->key[0]);
-  if (!rc) rc = C->get("key1", (size_t)n * k, &L->key[1]);
+  // both key arrays side by side: the leaf stage's position lists take them
+  int rc = C->get("keys01", 2 * (size_t)n * k, &L->key[0]);
+  L->key[1] = L->key[0] + (size_t)n * k;
   if (!rc) rc = C->get("id0", (size_t)n * k, &L->id[0]);
   if (!rc) rc = C->get("id1", (size_t)n * k, &L->id[1]);
   if (!rc) rc = C->get("flags0", (size_t)n * kw, &L->flags[0]);
@@ -458,6 +527,18 @@ bool leaf_filter_applies(const Layout& lay, int64_t n, int d, int k, int metric)
          (lay.maxleaf >= std::max(20, k + k / 2) && n * lay.maxleaf >= 800000 && d + 4 * k <= 256);
 }
 
+// The filter's scratch, of which a plain build has none to spare where memory is short.
+// Launches of fewer rows than 32,768 (eighth of a wave) would be slower than dense tiles.
+bool filter_scratch(knn_context* C, knn::FilterLeafArgs* f) {
+  const size_t rows = knn::filter_scratch_rows(*f);
+  if (!C->spare("Xp", (size_t)f->n * knn::umma_row_stride(f->d) * 2, &f->Xp) || !C->spare("norms_perm", (size_t)f->n, &f->np) ||
+      !C->spare("delta_perm", (size_t)f->n, &f->dp) || !C->spare("maxabs", 1, &f->maxabs) ||
+      !C->spare("leaf_survivors", (size_t)f->trees + 2, &f->survivors))
+    return false;
+  f->rows = (int64_t)C->spare_survivors(rows, std::min<size_t>(rows, 1 << 15), &f->surv, &f->count);
+  return f->rows > 0;
+}
+
 int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, int trees,
              const Layout& lay, int metric, const int32_t* perm, const float* norms, Lists* L,
              unsigned long long* counter, cudaStream_t st, knn::LaunchLog& log, int tile = 0,
@@ -489,7 +570,9 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
   a.fcount = lay.fcount;
   a.stream = st;
   a.pairs = pairs && lay.own_blocks && !lay.ftable;
-  if (sparse && metric != KNN_METRIC_COSINE && !lay.ftable) {
+  // sparse rows' scratch (dense tiles only)
+  auto sparse_scratch = [&]() -> int {
+    if (!sparse || metric == KNN_METRIC_COSINE || lay.ftable) return KNN_OK;
     a.lmax = 256 * ((dpad + 255) / 256);
     int rc = C->get("dmask", (size_t)lay.leaves * (dpad / 32 + 1), &a.dmask);
     if (!rc) rc = C->get("dlist", (size_t)lay.leaves * a.lmax, &a.dlist);
@@ -505,49 +588,50 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
       if (!rc)
         rc = C->get("tmask", (size_t)lay.leaves * ((lay.maxleaf + 31) / 32) * ((dpad + 31) / 32 + 1), &a.tmask);
     }
-    if (rc) return rc;
-  }
-  const bool filter = filter_ok && leaf_filter_applies(lay, n, d, k, metric);
+    return rc;
+  };
+  knn::FilterLeafArgs f{};
+  bool filter = filter_ok && leaf_filter_applies(lay, n, d, k, metric);
   // A first tree has no lists to filter by, so all its pairs would survive: it takes
   // dense tiles unless the bounding pass covers every leaf (six trees, 200,000 x 128,
   // leaf 360: 3.8 ms with the first tree filtered, 5.9 without; leaf 250, where that
   // pass does not apply: 15.8 against 6.5).
-  if (filter) a.trees = knn::umma_bounds_first_tree(lay.minleaf, k) ? 0 : 1;
-  int rc = a.trees > 0 ? knn::leaf_stage(a, log) : KNN_OK;
-  if (rc) return fail_cuda(cudaGetLastError(), "leaf stage launch");
-  if (!filter || trees <= a.trees) return KNN_OK;
-  knn::FilterLeafArgs f{};
-  f.X = X;
-  f.n = n;
-  f.d = d;
-  f.dpad = dpad;
-  f.k = k;
-  f.trees = trees;
-  f.first_tree = a.trees;
-  f.metric = metric;
-  f.segs = lay.segs;
-  f.leaves = lay.leaves;
-  f.maxleaf = lay.maxleaf;
-  f.tc_group = lay.tc_group_max;
-  f.perm = perm;
-  f.tree_inv = lay.tree_inv;
-  f.norms = norms;
-  f.rkey = a.rkey;
-  f.rid = a.rid;
-  f.pair_counter = counter;
-  f.give_up = C->filter_gives_up;
-  f.kev = kev;
-  f.stream = st;
-  rc = C->get("Xp", (size_t)n * knn::umma_row_stride(d) * 2, &f.Xp);
-  if (!rc) rc = C->get("norms_perm", (size_t)n, &f.np);
-  if (!rc) rc = C->get("delta_perm", (size_t)n, &f.dp);
-  if (!rc) rc = C->get("plist", (size_t)n * k, &f.plist);
-  const size_t srows = knn::filter_scratch_rows(f);
-  if (!rc) rc = C->get("survivors", srows * knn::umma_row_scratch_bytes(), &f.surv);
-  if (!rc) rc = C->get("surv_count", srows, &f.count);
-  if (!rc) rc = C->get("maxabs", 1, &f.maxabs);
-  if (!rc) rc = C->get("leaf_survivors", (size_t)trees + 2, &f.survivors);
+  f.first_tree = filter && knn::umma_bounds_first_tree(lay.minleaf, k) ? 0 : 1;
+  const bool every_tree = filter && f.first_tree == 0;
+  int rc = every_tree ? KNN_OK : sparse_scratch();
   if (rc) return rc;
+  if (filter) {
+    f.X = X;
+    f.n = n;
+    f.d = d;
+    f.dpad = dpad;
+    f.k = k;
+    f.trees = trees;
+    f.metric = metric;
+    f.segs = lay.segs;
+    f.leaves = lay.leaves;
+    f.maxleaf = lay.maxleaf;
+    f.tc_group = lay.tc_group_max;
+    f.perm = perm;
+    f.tree_inv = lay.tree_inv;
+    f.norms = norms;
+    f.rkey = a.rkey;
+    f.rid = a.rid;
+    f.plist = reinterpret_cast<int32_t*>(L->key[1 - L->cur]);  // the spare lists' keys
+    f.pair_counter = counter;
+    f.give_up = C->filter_gives_up;
+    f.kev = kev;
+    f.stream = st;
+    // without the scratch (or a tensor map) every tree takes dense tiles
+    filter = trees > f.first_tree && filter_scratch(C, &f) && knn::filter_map(&f);
+    if (!filter) C->done_with({"Xp", "norms_perm", "delta_perm", "maxabs", "leaf_survivors", "survivors", "surv_count"});
+  }
+  if (filter) a.trees = f.first_tree;
+  if (every_tree && !filter) rc = sparse_scratch();
+  if (rc) return rc;
+  rc = a.trees > 0 ? knn::leaf_stage(a, log) : KNN_OK;
+  if (rc) return fail_cuda(cudaGetLastError(), "leaf stage launch");
+  if (!filter) return KNN_OK;
   f.dense_tree = [&](int t, const unsigned long long* survivors, unsigned long long limit) {
     knn::LeafArgs one = a;
     one.first_tree = t;
@@ -613,20 +697,33 @@ int run_leaf_umma(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   a.rkey = L->key[L->cur];
   a.rid = L->id[L->cur];
   a.f16 = precision == KNN_PREC_F16_RERANK;
-  int rc = C->get("Xb", (size_t)n * ldr * 2, &a.Xb);
-  if (!rc) rc = C->get("Xp", (size_t)n * ldr * 2, &a.Xp);
-  if (!rc) rc = C->get("maxabs", 1, &a.maxabs);
-  if (!rc) rc = C->get("norms2", (size_t)n, &a.norms2);
-  if (!rc) rc = C->get("norms_perm", (size_t)n, &a.np);
   a.tree_inv = lay.tree_inv;
+  a.plist = reinterpret_cast<int32_t*>(L->key[0]);  // both key arrays hold 2 k >= kq positions a row; the lists come last
+  int rc = C->get("Xp", (size_t)n * ldr * 2, &a.Xp);
+  if (!rc) rc = C->get("maxabs", 1, &a.maxabs);
+  if (!rc) rc = C->get("norms_perm", (size_t)n, &a.np);
   if (!rc && trees > 1 && !a.tree_inv) rc = C->get("linv", (size_t)n, &a.inv);
-  if (!rc && trees > 1) rc = C->get("plist", (size_t)n * kq, &a.plist);
-  const size_t srows = knn::umma_scratch_rows(a);
-  if (!rc) rc = C->get("survivors", srows * knn::umma_row_scratch_bytes(), &a.surv);
-  if (!rc) rc = C->get("surv_count", srows, &a.surv_count);
   if (!rc) rc = C->get("akey", (size_t)n * kq, &a.akey);
   if (!rc) rc = C->get("aid", (size_t)n * kq, &a.aid);
   if (rc) return rc;
+  // where memory is short, first fewer rows a launch, then no operand copy in the rows' order
+  // (each tree converts the FP32 rows)
+  const size_t srows = knn::umma_scratch_rows(a);
+  const bool copy = C->spare("Xb", (size_t)n * ldr * 2, &a.Xb) && C->spare("norms2", (size_t)n, &a.norms2);
+  const size_t least = (size_t)knn::umma_block_rows(a);
+  if (copy) a.rows = (int64_t)C->spare_survivors(srows, least, &a.surv, &a.surv_count);
+  if (a.rows == 0) {
+    C->done_with({"Xb", "norms2"});
+    a.Xb = nullptr;
+    a.norms2 = nullptr;
+    a.rows = (int64_t)C->spare_survivors(srows, least, &a.surv, &a.surv_count);
+  }
+  if (a.rows == 0) {  // not even a block's
+    rc = C->get("survivors", least * knn::umma_row_scratch_bytes(), &a.surv);
+    if (!rc) rc = C->get("surv_count", least, &a.surv_count);
+    if (rc) return rc;
+    a.rows = (int64_t)least;
+  }
   rc = knn::leaf_stage_umma(a, log);
   if (rc == KNN_ERR_UNSUPPORTED) return fail(rc, "tensor-core leaf stage: unsupported shape");
   if (rc) return fail_cuda(cudaGetLastError(), "tensor-core leaf stage launch");
@@ -655,11 +752,12 @@ int prepare_filter(knn_context* C, const float* X, int64_t n, int d, int dpad, i
   a.metric = metric;
   a.norms = norms;
   a.stream = st;
-  int rc = C->get("Xp", (size_t)n * knn::prop_row_stride(d) * 2, &a.H);
-  if (!rc) rc = C->get("norms_perm", (size_t)n, &a.delta);
-  if (!rc) rc = C->get("maxabs", 1, &a.maxabs);
-  if (rc) return rc;
-  rc = knn::prop_prepare(a, log);
+  if (!C->spare("Xp", (size_t)n * knn::prop_row_stride(d) * 2, &a.H) || !C->spare("norms_perm", (size_t)n, &a.delta) ||
+      !C->spare("maxabs", 1, &a.maxabs)) {  // every key exact instead
+    C->done_with({"Xp", "norms_perm", "maxabs"});
+    return KNN_OK;
+  }
+  const int rc = knn::prop_prepare(a, log);
   if (rc) return fail_cuda(cudaGetLastError(), "propagation rows launch");
   F->H = a.H;
   F->delta = a.delta;
@@ -912,16 +1010,16 @@ int learn_network(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   if (!rc)
     rc = run_leaf(C, Xs, ns, d, dpad, gk, kMlpGraphTrees, single_layout(ns, T.depth), metric, T.perm, norms, &L,
                   nullptr, st, log);
+  int32_t* graph = nullptr;
+  float* gdist = nullptr;
+  if (!rc) rc = C->get("mlp_graph", (size_t)ns * gk, &graph);
+  if (!rc) rc = C->get("mlp_gdist", (size_t)ns * gk, &gdist);
   PropFilter F;
   if (!rc) rc = prepare_filter(C, Xs, ns, d, dpad, gk, metric, norms, st, &F, log);
   for (int p = 0; !rc && p < kMlpGraphProps; ++p)
     rc = run_prop(Xs, ns, d, dpad, gk, metric, norms, T.perm, &L, true, nullptr, st, log, F);
   if (rc) return rc;
-  int32_t* graph = nullptr;
-  float* gdist = nullptr;
-  rc = C->get("mlp_graph", (size_t)ns * gk, &graph);
-  if (!rc) rc = C->get("mlp_gdist", (size_t)ns * gk, &gdist);
-  if (rc) return rc;
+  C->done_with({"Xp", "norms_perm", "maxabs"});
   knn::launch_finalize(L.key[L.cur], L.id[L.cur], ns, gk, metric, gdist, graph, st);
   log.add();
 
@@ -1001,6 +1099,7 @@ int enter_device(knn_context** ctx, const knn_options& o) {
     return fail(KNN_ERR_ARGS, "context device differs from options.device");
   }
   KNN_CK(cudaSetDevice((*ctx)->device));
+  ++(*ctx)->call;
   return KNN_OK;
 }
 
@@ -1086,6 +1185,13 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
   Lists L;
   rc = get_lists(C, n, k, &L);
   if (rc) return rc;
+  float* dd = out_dist;
+  int32_t* di = out_idx;
+  if (!o.outputs_on_device) {
+    rc = C->get("out_dist", (size_t)n * k, &dd);
+    if (!rc) rc = C->get("out_idx", (size_t)n * k, &di);
+    if (rc) return rc;
+  }
   int* err_flag = C->err_words;
   rc = reset_error_word(C, o.precision, st);
   if (rc) return rc;
@@ -1145,13 +1251,6 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
   if (timed) KNN_CK(cudaEventRecord(C->ev[4], st));
 
   // Finalise into the caller's buffers (or staging, then copy to the host).
-  float* dd = out_dist;
-  int32_t* di = out_idx;
-  if (!o.outputs_on_device) {
-    rc = C->get("out_dist", (size_t)n * k, &dd);
-    if (!rc) rc = C->get("out_idx", (size_t)n * k, &di);
-    if (rc) return rc;
-  }
   // raw keys: no sqrt (the TAXICAB transform is the identity)
   knn::launch_finalize(L.key[L.cur], L.id[L.cur], n, k, o.raw_keys ? KNN_METRIC_TAXICAB : metric, dd, di, st);
   log.add();
@@ -1379,6 +1478,7 @@ int batch_impl(knn_context* C, const knn_dataset* sets, int count, int32_t k, in
   float stage_ms[3] = {0, 0, 0};
 
   for (auto& kv : by_d) {
+    ++C->call;  // the last group's scratch is done with
     const BatchGroup g = make_group(sets, kv.second, kv.first, leaf);
     for (const auto& e : g.hsegs)
       if (e.depth > 30) return fail(KNN_ERR_ARGS, "tree too deep (n / leaf too large)");
@@ -1589,6 +1689,16 @@ int knn_test_fail_next_tile_wait(knn_context* ctx) {
   return KNN_OK;
 }
 
+int knn_test_limit_scratch(knn_context* ctx, int64_t bytes) {
+  if (bytes < 0) return fail(KNN_ERR_ARGS, "negative limit");
+  knn_options o;
+  knn_default_options(&o);
+  int rc = enter_device(&ctx, o);
+  if (rc) return rc;
+  ctx->scratch_limit = bytes;
+  return KNN_OK;
+}
+
 int knn_build(const void* points, int64_t n, int32_t d, int32_t k, int32_t trees, int32_t leaf,
               int32_t props, int32_t metric, uint64_t seed, int32_t* out_idx, float* out_dist) {
   return knn_build_ex(nullptr, points, n, d, k, trees, leaf, props, metric, seed, out_idx,
@@ -1740,16 +1850,16 @@ int knn_propagate_step(knn_context* ctx, const float* points, int64_t n, int32_t
   if (rc) return rc;
   KNN_CK(cudaMemcpyAsync(L.key[0], key_in, sizeof(float) * (size_t)n * k, cudaMemcpyHostToDevice, st));
   KNN_CK(cudaMemcpyAsync(L.id[0], idx_in, sizeof(int32_t) * (size_t)n * k, cudaMemcpyHostToDevice, st));
-  PropFilter F;
-  rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
-  if (rc) return rc;
-  rc = run_prop(P.X, n, d, P.dpad, k, metric, norms, nullptr, &L, false, nullptr, st, log, F);
-  if (rc) return rc;
   int32_t* di = nullptr;
   rc = ctx->get("out_idx", (size_t)n * k, &di);
   if (rc) return rc;
   float* dd = nullptr;
   rc = ctx->get("out_dist", (size_t)n * k, &dd);
+  if (rc) return rc;
+  PropFilter F;
+  rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+  if (rc) return rc;
+  rc = run_prop(P.X, n, d, P.dpad, k, metric, norms, nullptr, &L, false, nullptr, st, log, F);
   if (rc) return rc;
   // ids without flag bits; keys as they are
   knn::launch_finalize(L.key[L.cur], L.id[L.cur], n, k, KNN_METRIC_TAXICAB, dd, di, st);

@@ -146,15 +146,16 @@ struct UmmaLeafArgs {
   const int32_t* perm;   // [trees][n]
   const float* norms;    // [n] FP32 norms (COSINE) or null
   bool f16;              // operands FP16 (else BF16)
-  void* Xb;              // [n][umma_row_stride(d)] 16-bit operand scratch
+  void* Xb;              // [n][umma_row_stride(d)] 16-bit operand scratch, or null: each tree converts X
   void* Xp;              // the same in a tree's order
   unsigned int* maxabs;  // [1] scratch: largest |x| (FP16 EUCLIDEAN row scale)
-  float* norms2;         // [n] scratch
+  float* norms2;         // [n] scratch (with Xb)
   float* np;             // [n] scratch: norms2 in a tree's order
   const int32_t* tree_inv;  // [trees][n] the trees' inverse orders, or null: computed into inv
   int32_t* inv;          // [n] scratch (tree_inv null, several trees)
-  void* surv;            // [umma_scratch_rows(...)][umma_row_scratch_bytes()] scratch: the tiles' survivors
-  uint32_t* surv_count;  // [umma_scratch_rows(...)]
+  int64_t rows;          // rows of the survivor scratch: umma_scratch_rows(...), or fewer (a block's at least)
+  void* surv;            // [rows][umma_row_scratch_bytes()] scratch: the tiles' survivors
+  uint32_t* surv_count;  // [rows]
   int32_t* plist;        // [n][kq] scratch: positions of the lists' entries (several trees)
   cudaEvent_t* kev;      // [2 * trees] events around each tree's tile kernel, or null
   uint32_t* akey;        // [n][kq] scratch: approximate lists (ordered keys and ids)
@@ -169,6 +170,7 @@ struct UmmaLeafArgs {
 };
 int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log);
 size_t umma_scratch_rows(const UmmaLeafArgs& a);  // from the shape fields
+int umma_block_rows(const UmmaLeafArgs& a);       // rows of one block
 size_t umma_row_scratch_bytes();
 // Elements per row of the 16-bit operand copies: whole 16-byte units.
 inline int umma_row_stride(int d) { return (d + 7) & ~7; }
@@ -192,8 +194,9 @@ struct FilterLeafArgs {
   float* np;                // [n] scratch
   float* dp;                // [n] scratch
   int32_t* plist;           // [n][k] scratch
-  void* surv;               // [filter_scratch_rows(...)][umma_row_scratch_bytes()] scratch
-  uint32_t* count;          // [filter_scratch_rows(...)] scratch
+  int64_t rows;             // rows of the survivor scratch: filter_scratch_rows(...), or fewer
+  void* surv;               // [rows][umma_row_scratch_bytes()] scratch
+  uint32_t* count;          // [rows] scratch
   unsigned int* maxabs;
   // [trees + 2] scratch: a zero, each tree's survivors, and the words of waits that gave up
   unsigned long long* survivors;
@@ -201,11 +204,13 @@ struct FilterLeafArgs {
   std::function<int(int t, const unsigned long long* survivors, unsigned long long limit)> dense_tree;
   unsigned long long* pair_counter;
   bool give_up;             // test hook: as if every wait gave up
+  alignas(64) unsigned char map[128];  // filter_map
   cudaEvent_t* kev;
   cudaStream_t stream;
 };
 // The bounding pass covers every leaf of at least minleaf points that is its own block.
 bool umma_bounds_first_tree(int64_t minleaf, int k);
+bool filter_map(FilterLeafArgs* a);  // the tensor map of Xp; false where the driver refuses it
 int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log);
 size_t filter_scratch_rows(const FilterLeafArgs& a);  // from the shape fields
 

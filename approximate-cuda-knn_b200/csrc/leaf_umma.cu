@@ -48,6 +48,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "knn_internal.cuh"
 #include "knn_kernels.cuh"
@@ -65,7 +66,10 @@ constexpr int kRing = 4;              // candidate boxes in flight (at least a t
 constexpr int kCap = 192;
 constexpr int kFlushAt = kCap - kTN;  // a fuller buffer could not take another tile
 constexpr int kFlushMin = 24;         // rows merged along when one row's buffer is full
-constexpr int64_t kChunkRows = 1 << 19;  // rows (of whole blocks) per launch: bounds the survivor scratch
+// Rows (of whole blocks) per launch: bounds the survivor scratch, 1.5 KB a row, at 805 MB.  Half as
+// many cost 6 % of the headline build (22.7 -> 24.0 ms) and 5 % at 10M rows, a quarter 14 %: each
+// launch ends in a tail.  Less is used where memory is short.
+constexpr int64_t kChunkRows = 1 << 19;
 constexpr uint32_t kOverflow = 0xFFFFFFFFu;  // FP32 filter: more survivors than the buffer holds, evaluate the block
 constexpr uint32_t kListed = 0x80000000u;  // count flag (first tree): the row's list was already written
 constexpr int kBand = 1024;           // block columns covered by the listed-column bitmap at a time
@@ -1335,13 +1339,15 @@ __device__ __forceinline__ float from_operand(uint16_t b, bool f16) {
 // values (EUCLIDEAN).  FP16 EUCLIDEAN rows are first multiplied by the power
 // of two 2^e that brings the largest |x| (maxabs) into [2^14, 2^15), inside
 // the FP16 range: a power-of-two scale is exact, scales every key of the tile
-// stage by the same 2^2e and so keeps its ranking (the re-rank uses X).
+// stage by the same 2^2e and so keeps its ranking (the re-rank uses X).  With perm,
+// output row i is row perm[i].
 __global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int dpad, int ldr, int metric, bool f16,
                              const unsigned int* __restrict__ maxabs, const float* __restrict__ norms,
-                             uint16_t* __restrict__ Xb, float* __restrict__ norms2) {
-  const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+                             const int32_t* __restrict__ perm, uint16_t* __restrict__ Xb, float* __restrict__ norms2) {
+  const int64_t out = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (row >= n) return;
+  if (out >= n) return;
+  const int64_t row = perm ? perm[out] : out;
   float scale = 1.f;
   if (metric == KNN_METRIC_COSINE) {
     const float nr = norms[row];
@@ -1360,13 +1366,13 @@ __global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int 
   for (int c = lane; c < ldr; c += 32) {
     const float v = c < d ? X[(size_t)row * dpad + c] : 0.f;
     const uint16_t b = to_operand(__fmul_rn(v, scale), f16);
-    Xb[(size_t)row * ldr + c] = b;
+    Xb[(size_t)out * ldr + c] = b;
     const float f = from_operand(b, f16);
     s = __fmaf_rn(f, f, s);
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, off));
-  if (lane == 0) norms2[row] = s;
+  if (lane == 0) norms2[out] = s;
 }
 
 // A tree's order: Xp[i] = Xb[perm[i]], np[i] = norms2[perm[i]]; one thread per
@@ -1496,15 +1502,15 @@ bool operand_map(const void* Xp, int64_t n, int ldr, bool f16, CUtensorMap* map)
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A tree's tiles, kChunkRows rows at a time, each chunk followed by its merge
+// A tree's tiles, `rows` rows at a time, each chunk followed by its merge
 // (BOUND: into the exact lists rkey / rid).
 template <int METRIC, bool BOUND, bool FIRST, bool PRE, int NCH, int QT>
-void launch_tc(const CUtensorMap& map, LeafTcArgs t, int64_t blocks, float* rkey, uint32_t* rid, cudaStream_t st,
-               LaunchLog& log) {
+void launch_tc(const CUtensorMap& map, LeafTcArgs t, int64_t blocks, int64_t rows, float* rkey, uint32_t* rid,
+               cudaStream_t st, LaunchLog& log) {
   const size_t smem = leaf_tc_smem<NCH, QT>();
   cudaFuncSetAttribute(k_leaf_tc<METRIC, BOUND, FIRST, PRE, NCH, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
-  const int64_t chunk = kChunkRows / (kBM * QT);
+  const int64_t chunk = rows / (kBM * QT);
   for (t.block0 = 0; t.block0 < blocks; t.block0 += chunk) {
     const unsigned grid = (unsigned)std::min(chunk, blocks - t.block0);
     k_leaf_tc<METRIC, BOUND, FIRST, PRE, NCH, QT><<<grid, 64 + 128 * QT, smem, st>>>(map, t);
@@ -1523,21 +1529,21 @@ void launch_tc(const CUtensorMap& map, LeafTcArgs t, int64_t blocks, float* rkey
   }
 }
 template <int METRIC, bool BOUND, bool FIRST, bool PRE>
-void launch_tc_tiles(int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks, float* rkey,
-                     uint32_t* rid, cudaStream_t st, LaunchLog& log) {
-  if (qt == 2 && nch == 1) launch_tc<METRIC, BOUND, FIRST, PRE, 1, 2>(map, t, blocks, rkey, rid, st, log);
-  else if (qt == 2) launch_tc<METRIC, BOUND, FIRST, PRE, 2, 2>(map, t, blocks, rkey, rid, st, log);
-  else if (nch == 1) launch_tc<METRIC, BOUND, FIRST, PRE, 1, 1>(map, t, blocks, rkey, rid, st, log);
-  else if (nch == 2) launch_tc<METRIC, BOUND, FIRST, PRE, 2, 1>(map, t, blocks, rkey, rid, st, log);
-  else if (nch == 3) launch_tc<METRIC, BOUND, FIRST, PRE, 3, 1>(map, t, blocks, rkey, rid, st, log);
-  else launch_tc<METRIC, BOUND, FIRST, PRE, 4, 1>(map, t, blocks, rkey, rid, st, log);
+void launch_tc_tiles(int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks, int64_t rows,
+                     float* rkey, uint32_t* rid, cudaStream_t st, LaunchLog& log) {
+  if (qt == 2 && nch == 1) launch_tc<METRIC, BOUND, FIRST, PRE, 1, 2>(map, t, blocks, rows, rkey, rid, st, log);
+  else if (qt == 2) launch_tc<METRIC, BOUND, FIRST, PRE, 2, 2>(map, t, blocks, rows, rkey, rid, st, log);
+  else if (nch == 1) launch_tc<METRIC, BOUND, FIRST, PRE, 1, 1>(map, t, blocks, rows, rkey, rid, st, log);
+  else if (nch == 2) launch_tc<METRIC, BOUND, FIRST, PRE, 2, 1>(map, t, blocks, rows, rkey, rid, st, log);
+  else if (nch == 3) launch_tc<METRIC, BOUND, FIRST, PRE, 3, 1>(map, t, blocks, rows, rkey, rid, st, log);
+  else launch_tc<METRIC, BOUND, FIRST, PRE, 4, 1>(map, t, blocks, rows, rkey, rid, st, log);
 }
 template <int METRIC, bool BOUND>
 void launch_tc_tree(bool first, bool pre, int qt, int nch, const CUtensorMap& map, const LeafTcArgs& t, int64_t blocks,
-                    float* rkey, uint32_t* rid, cudaStream_t st, LaunchLog& log) {
-  if (first) launch_tc_tiles<METRIC, BOUND, true, true>(qt, nch, map, t, blocks, rkey, rid, st, log);
-  else if (pre) launch_tc_tiles<METRIC, BOUND, false, true>(qt, nch, map, t, blocks, rkey, rid, st, log);
-  else launch_tc_tiles<METRIC, BOUND, false, false>(qt, nch, map, t, blocks, rkey, rid, st, log);
+                    int64_t rows, float* rkey, uint32_t* rid, cudaStream_t st, LaunchLog& log) {
+  if (first) launch_tc_tiles<METRIC, BOUND, true, true>(qt, nch, map, t, blocks, rows, rkey, rid, st, log);
+  else if (pre) launch_tc_tiles<METRIC, BOUND, false, true>(qt, nch, map, t, blocks, rows, rkey, rid, st, log);
+  else launch_tc_tiles<METRIC, BOUND, false, false>(qt, nch, map, t, blocks, rows, rkey, rid, st, log);
 }
 
 }  // namespace
@@ -1567,6 +1573,7 @@ size_t umma_scratch_rows(const UmmaLeafArgs& a) {
   for (int t = 0; a.ftable && t < a.trees; ++t) leaves = std::max(leaves, a.fcount[t]);
   return (size_t)std::min<int64_t>(kChunkRows, leaves * s.qtiles * (kBM * s.qt));
 }
+int umma_block_rows(const UmmaLeafArgs& a) { return kBM * tc_shape(a.d, a.maxleaf, a.tc_group).qt; }
 size_t umma_row_scratch_bytes() { return kCap * sizeof(uint2); }
 
 int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
@@ -1582,9 +1589,12 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
     log.add();
   }
   const int ldr = umma_row_stride(a.d);
-  k_to_operand<<<(unsigned)((a.n * 32 + 255) / 256), 256, 0, st>>>(a.X, a.n, a.d, a.dpad, ldr, a.metric, a.f16,
-                                                                    a.maxabs, a.norms, Xb, a.norms2);
-  log.add();
+  auto convert = [&](const int32_t* perm, uint16_t* rows, float* norms2) {
+    k_to_operand<<<(unsigned)((a.n * 32 + 255) / 256), 256, 0, st>>>(a.X, a.n, a.d, a.dpad, ldr, a.metric, a.f16,
+                                                                      a.maxabs, a.norms, perm, rows, norms2);
+    log.add();
+  };
+  if (Xb) convert(nullptr, Xb, a.norms2);
   CUtensorMap map;
   if (!operand_map(a.Xp, a.n, ldr, a.f16, &map)) return KNN_ERR_CUDA;
   const int64_t leaves = a.leaves;
@@ -1622,9 +1632,13 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
       continue;
     }
     const int64_t blocks = tleaves * t.qtiles;
-    k_permute_operand<<<(unsigned)((a.n * units + 255) / 256), 256, 0, st>>>(
-        reinterpret_cast<const uint4*>(Xb), a.norms2, t.perm, a.n, units, static_cast<uint4*>(a.Xp), a.np);
-    log.add();
+    if (Xb) {
+      k_permute_operand<<<(unsigned)((a.n * units + 255) / 256), 256, 0, st>>>(
+          reinterpret_cast<const uint4*>(Xb), a.norms2, t.perm, a.n, units, static_cast<uint4*>(a.Xp), a.np);
+      log.add();
+    } else {
+      convert(t.perm, static_cast<uint16_t*>(a.Xp), a.np);
+    }
     if (tr > 0) {
       const int32_t* inv = a.tree_inv ? a.tree_inv + (size_t)tr * a.n : a.inv;
       if (!a.tree_inv) {
@@ -1638,9 +1652,9 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
     if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
     const bool pre = tr < kPrepassTrees && a.maxleaf >= kPrepassMin;
     if (a.metric == KNN_METRIC_EUCLIDEAN)
-      launch_tc_tree<KNN_METRIC_EUCLIDEAN, false>(tr == 0, pre, qt, nch, map, t, blocks, nullptr, nullptr, st, log);
+      launch_tc_tree<KNN_METRIC_EUCLIDEAN, false>(tr == 0, pre, qt, nch, map, t, blocks, a.rows, nullptr, nullptr, st, log);
     else
-      launch_tc_tree<KNN_METRIC_COSINE, false>(tr == 0, pre, qt, nch, map, t, blocks, nullptr, nullptr, st, log);
+      launch_tc_tree<KNN_METRIC_COSINE, false>(tr == 0, pre, qt, nch, map, t, blocks, a.rows, nullptr, nullptr, st, log);
     if (a.kev) cudaEventRecord(a.kev[2 * tr + 1], st);
   }
   const size_t rsm = (size_t)8 * (a.dpad + 32 * 64 + 32) * sizeof(float);
@@ -1666,6 +1680,14 @@ size_t filter_scratch_rows(const FilterLeafArgs& a) {
 // width reach 1.25 k at every size from minleaf on if they do at 256.
 bool umma_bounds_first_tree(int64_t minleaf, int k) { return minleaf >= kPrepassMin && 8 * (k + k / 4) <= kPrepassMin; }
 
+bool filter_map(FilterLeafArgs* a) {
+  CUtensorMap map;
+  if (!operand_map(a->Xp, a->n, umma_row_stride(a->d), true, &map)) return false;
+  static_assert(sizeof(map) == sizeof(a->map), "tensor map");
+  memcpy(a->map, &map, sizeof(map));
+  return true;
+}
+
 int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   const int nch = (a.d + kKC - 1) / kKC;
   if (nch > 4 || a.k > 32 || a.metric == KNN_METRIC_TAXICAB) return KNN_ERR_UNSUPPORTED;
@@ -1679,7 +1701,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
     log.add();
   }
   CUtensorMap map;
-  if (!operand_map(a.Xp, a.n, ldr, true, &map)) return KNN_ERR_CUDA;
+  memcpy(&map, a.map, sizeof(map));
   LeafTcArgs t{};
   t.Xp = static_cast<const uint16_t*>(a.Xp);
   t.np = a.np;
@@ -1727,7 +1749,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
       t.plist = a.plist;
     }
     const bool pre = tr < kPrepassTrees && a.maxleaf >= kPrepassMin;
-    launch_tc_tree<KNN_METRIC_EUCLIDEAN, true>(tr == 0, pre, shape.qt, nch, map, t, blocks, a.rkey, a.rid, st, log);
+    launch_tc_tree<KNN_METRIC_EUCLIDEAN, true>(tr == 0, pre, shape.qt, nch, map, t, blocks, a.rows, a.rkey, a.rid, st, log);
     const int rc = a.dense_tree(tr, t.survivors, t.survivor_limit);
     if (rc) return rc;
     if (a.kev) cudaEventRecord(a.kev[2 * tr + 1], st);

@@ -174,7 +174,9 @@ int knn_device_capability(int32_t device, int32_t* major, int32_t* minor);
  * Returns NULL on failure (see knn_last_error). */
 knn_context* knn_context_create(int32_t device);
 void knn_context_destroy(knn_context* ctx);
-/* Bytes of device scratch the context currently holds. */
+/* Bytes of device scratch the context currently holds.  Where device memory is
+ * short, a call first gives back the scratch of earlier calls, then does without
+ * what only makes it faster (16-bit rows, the leaf filter's survivor lists). */
 int64_t knn_context_scratch_bytes(const knn_context* ctx);
 
 /* Outcome of the context's asynchronous calls.  A build given a caller stream,
@@ -194,6 +196,11 @@ int knn_context_status(knn_context* ctx, void* stream);
  * are only a filter, takes dense FP32 tiles instead and succeeds.  One-shot; the
  * build after it runs normally. */
 int knn_test_fail_next_tile_wait(knn_context* ctx);
+
+/* Test hook: device scratch allocations of `ctx` (NULL: the thread's default
+ * context) that would take it past `bytes` fail as if the device were full; 0
+ * lifts the limit. */
+int knn_test_limit_scratch(knn_context* ctx, int64_t bytes);
 
 /*
  * knn_build -- the drop-in call.  Replaces EuclideanDistanceMatrixGPU::initialize
