@@ -742,8 +742,8 @@ struct PropFilter {
 // 16-bit rows for the steps that follow.  They take the tensor-core leaf
 // stage's operand buffer, which is done with by then and has the same size.
 int prepare_filter(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, int metric, const float* norms,
-                   cudaStream_t st, PropFilter* F, knn::LaunchLog& log) {
-  if (!knn::prop_filter_applies(k, d)) return KNN_OK;
+                   bool half, cudaStream_t st, PropFilter* F, knn::LaunchLog& log) {
+  if (!knn::prop_filter_applies(k, d) || !knn::prop_filter_pays(k, d, metric, half)) return KNN_OK;
   knn::PropPrep a{};
   a.X = X;
   a.n = n;
@@ -1015,7 +1015,7 @@ int learn_network(knn_context* C, const float* X, int64_t n, int d, int dpad, in
   if (!rc) rc = C->get("mlp_graph", (size_t)ns * gk, &graph);
   if (!rc) rc = C->get("mlp_gdist", (size_t)ns * gk, &gdist);
   PropFilter F;
-  if (!rc) rc = prepare_filter(C, Xs, ns, d, dpad, gk, metric, norms, st, &F, log);
+  if (!rc) rc = prepare_filter(C, Xs, ns, d, dpad, gk, metric, norms, false, st, &F, log);
   for (int p = 0; !rc && p < kMlpGraphProps; ++p)
     rc = run_prop(Xs, ns, d, dpad, gk, metric, norms, T.perm, &L, true, nullptr, st, log, F);
   if (rc) return rc;
@@ -1236,7 +1236,7 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
   if (rc) return rc;
   if (timed) KNN_CK(cudaEventRecord(C->ev[3], st));
   PropFilter F;
-  if (props > 0) rc = prepare_filter(C, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+  if (props > 0) rc = prepare_filter(C, P.X, n, d, P.dpad, k, metric, norms, P.Xh != nullptr, st, &F, log);
   if (rc) return rc;
   if (tune_prop) {
     rc = finish_prop_tuning(C, o, P.X, n, d, P.dpad, k, metric, norms, T.perm, &L, lay.maxleaf, st, F, &sh);
@@ -1431,7 +1431,7 @@ int group_compute(knn_context* C, const BatchGroup& g, int k, int trees, int pro
   if (rc) return rc;
   if (stage_events) KNN_CK(cudaEventRecord(C->ev[3], st));
   PropFilter F;
-  if (props > 0) rc = prepare_filter(C, X, g.ntot, g.d, g.dpad, k, metric, norms, st, &F, log);
+  if (props > 0) rc = prepare_filter(C, X, g.ntot, g.d, g.dpad, k, metric, norms, false, st, &F, log);
   if (rc) return rc;
   if (tune_prop) {
     rc = finish_prop_tuning(C, o, X, g.ntot, g.d, g.dpad, k, metric, norms, T.perm, &L, lay.maxleaf, st, F, &sh);
@@ -1857,7 +1857,7 @@ int knn_propagate_step(knn_context* ctx, const float* points, int64_t n, int32_t
   rc = ctx->get("out_dist", (size_t)n * k, &dd);
   if (rc) return rc;
   PropFilter F;
-  rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+  rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, false, st, &F, log);
   if (rc) return rc;
   rc = run_prop(P.X, n, d, P.dpad, k, metric, norms, nullptr, &L, false, nullptr, st, log, F);
   if (rc) return rc;
@@ -2011,7 +2011,7 @@ int knn_propagate_range(knn_context* ctx, const void* points, int64_t n, int32_t
   if (r1 > r0) {
     // the filter's rows take one pass over all points: not for a small range
     PropFilter F;
-    if ((r1 - r0) * 8 >= n) rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, st, &F, log);
+    if ((r1 - r0) * 8 >= n) rc = prepare_filter(ctx, P.X, n, d, P.dpad, k, metric, norms, P.Xh != nullptr, st, &F, log);
     if (rc) return rc;
     knn::PropArgs a{};
     a.X = P.X;

@@ -217,6 +217,7 @@ size_t filter_scratch_rows(const FilterLeafArgs& a);  // from the shape fields
 // 16-bit rows for the propagation's candidate filter (propagate.cu).
 inline int prop_row_stride(int d) { return (d + 7) & ~7; }
 bool prop_filter_applies(int k, int d);
+bool prop_filter_pays(int k, int d, int metric, bool half);  // half: the exact kernel gathers FP16 rows
 struct PropPrep {
   const float* X;
   int64_t n;

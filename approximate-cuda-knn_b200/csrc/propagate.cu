@@ -16,8 +16,9 @@
 // Up to 1024 dims k_propagate_filtered, below, first rejects the candidates that
 // cannot enter from 16-bit rows with rigorous bounds, and computes exact keys only
 // for the rest: the same result.  k_propagate, every key exact, remains for longer
-// rows, lists too long for the filter's shared memory, and ranges so small that
-// preparing all points' 16-bit rows would cost more than the range.
+// rows, lists too long for the filter's shared memory, shapes where it is the faster one
+// (prop_filter_pays), and ranges so small that preparing all points' 16-bit rows
+// would cost more than the range.
 // "New" flags: a pair (a, j) is skipped when a was already in N(i) and j already
 // in N(a) before the previous step.  Such a j was a candidate of i in that step
 // and lost to k better entries (or is listed), and N(i) only improves, so it
@@ -741,8 +742,40 @@ static void launch_filtered(const PropArgs& a, int kpl, int hbits, size_t wb, in
 #undef KNN_FILT_LAUNCH
 }
 
+// Blocks per SM of k_propagate with its warps per block (one row-slice buffer).
+static int exact_blocks(int k, int d, int* wpb) {
+  const size_t wb = prop_warp_bytes(k, d, 1);
+  *wpb = (int)std::min<size_t>(kPropMaxWarps, kPropSmemBudget / wb);
+  return *wpb < 1 ? 0 : std::max(1, (int)((220 * 1024) / (wb * *wpb)));
+}
+
 bool prop_filter_applies(int k, int d) {
   return d <= kFiltMaxDim && filt_warp_bytes(k, d) <= kPropSmemBudget;
+}
+
+// Whether the filter is the faster one.  Where k_propagate keeps two blocks of eight warps per
+// SM (lists up to 15, fewer from 576 dims on), it is not always: it reads FP16 input at
+// half the bytes too, COSINE keys cost it one instruction per dim, and the filter's lanes
+// read power-of-two widths (`idle` = width over dims).  Two steps, 100,000 points, 64 clusters,
+// filter against exact, EUCLIDEAN / COSINE, k = 8: 136 dims 1.14 / 1.18, 192 1.10 / 1.18, 208
+// 0.96 / 1.03, 256 0.95 / 1.05, 300 1.18 / 1.31, 384 1.05 / 1.21, 448 0.98 / 1.15, 512 0.91 / 1.10,
+// 520 1.27 / 1.50, 784 1.00 / 1.14, 900 0.89 / 1.24, 1,000 0.50 / 0.82 (one block); FP16 input
+// 96 dims 0.98, 136 1.24, 256 1.17, 520 1.61.  k = 4: 136 0.99 / 1.01, 340 0.95 / 1.09, 520
+// 1.07 / 1.27, FP16 136 0.99, 340 1.16.  Tiny rows
+// and lists leave nothing to reject: k = 5, 8 dims 1.44 / 1.20, 16 dims 1.07 / 0.91; k = 3, 40 dims
+// 1.43 / 1.29, 72 0.92 / 0.85.  One block per SM: 0.29 to 0.99.
+bool prop_filter_pays(int k, int d, int metric, bool half) {
+  if ((k <= 5 && d <= 8) || (k <= 3 && d <= 40)) return false;
+  int wpb;
+  const bool cosine = metric == KNN_METRIC_COSINE;
+  const int shortest = d > 256 && (half || cosine) ? 4 : 5;  // shorter lists: the filter
+  if (d <= 128 || k < shortest || exact_blocks(k, d, &wpb) < 2 || wpb < kPropMaxWarps) return true;
+  if (half) return false;
+  int width = 256;
+  while (width < d) width *= 2;
+  const double idle = (double)width / d;
+  if (cosine) return idle < (d <= 256 ? 1.33 : 1.12);
+  return d <= 256 ? idle < 1.33 || k < 6 : idle < 1.45;
 }
 
 int prop_prepare(const PropPrep& a, LaunchLog& log) {
@@ -785,9 +818,8 @@ int propagate_step(const PropArgs& a, LaunchLog& log) {
     return cudaPeekAtLastError() == cudaSuccess ? KNN_OK : KNN_ERR_CUDA;
   }
   size_t wb = prop_warp_bytes(a.k, a.d, 1);
-  int wpb = (int)(kPropSmemBudget / wb);
-  if (wpb > kPropMaxWarps) wpb = kPropMaxWarps;
-  if (wpb < 1) return KNN_ERR_UNSUPPORTED;
+  int wpb;
+  if (exact_blocks(a.k, a.d, &wpb) < 1) return KNN_ERR_UNSUPPORTED;
   if (a.warps > 0 && a.warps < wpb) wpb = a.warps;  // a tuned block size (results identical)
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
