@@ -211,7 +211,10 @@ __device__ __forceinline__ float exact_limit(double tk, double g, int d, double 
 //
 // Data whose k-th keys tie with much of the set (copies of few points) would queue
 // most pairs, at about 2.5 times k_exact's cost per pair: a block whose warp has queued a
-// third of its pairs marks itself for k_exact and ends.
+// third of its pairs, past what open lists take (8 k (1 + ln(candidates / k)) pairs, a first
+// tile's 1,024 at most), marks itself for k_exact and ends.  2,000 queries x 100,000 x 64, all
+// rows equal, against k_exact alone: k = 16 1.35 with an allowance of 4,096 pairs, 1.00 now, k = 40 1.59
+// and 1.2; with 512 + 8 k pairs ordinary data gave up too (k = 100: 37.8 -> 47 ms).
 template <int METRIC, int KPL>
 __global__ void __launch_bounds__(256, KPL == 1 ? 2 : 1)
     k_exact_filtered(const float* __restrict__ X, int64_t n, int d, int dpad, bool vec, int k,
@@ -426,7 +429,7 @@ __global__ void __launch_bounds__(256, KPL == 1 ? 2 : 1)
     seen += 8 * kFC;
     // every warp sees the same verdict; the barrier also keeps the next tile's
     // norms from overwriting those that a late warp still reads
-    if (__syncthreads_or(taken > 4096 + seen / 3)) {
+    if (__syncthreads_or(taken > (KPL <= 2 ? 512 : 1024) + 16 * k + seen / 3)) {
       if (tid == 0) part_idx[((size_t)blockIdx.y * nq + q0) * k] = kRedoMark;
       return;
     }
