@@ -1,6 +1,8 @@
 """Propagation with and without the candidate filter: shapes on either side of the rule that chooses between them give the
-CPU restatement's lists, in FP32 and from FP16 rows."""
+CPU restatement's lists, in FP32 and from FP16 rows, and the ranges of a sharded step take one route."""
 from __future__ import annotations
+
+import ctypes
 
 import numpy as np
 import pytest
@@ -21,3 +23,41 @@ def test_either_side(oracle, metric, d, k):
         oi, od = oracle.knn_build(y.astype(np.float32), k, 2, max(24, 2 * k), 2, metric, seed=1)
         np.testing.assert_array_equal(gi, oi)
         np.testing.assert_array_equal(gd.view(np.uint32), od.view(np.uint32))
+
+
+@pytest.mark.parametrize("world", [3, 7, 8, 9, 12])
+def test_ranges_of_a_step_take_one_route(world):
+    """Ranges of an even split differ by a point; the filter's rows are scratch, so the route shows in the bytes held."""
+    torch = pytest.importorskip("torch")
+    acknn = load_package()
+    lib = acknn.load_library()
+    n, d, k = 4003, 24, 16
+    x = torch.from_numpy(acknn.workloads.gaussian_mixture(n, d, 8, seed=1)).cuda()
+    ctx = acknn.Context(0)
+    idx = torch.empty((n, k), dtype=torch.int32, device="cuda")
+    key = torch.empty((n, k), dtype=torch.float32, device="cuda")
+    opt = acknn.default_options(points_on_device=1, outputs_on_device=1, raw_keys=1)
+    assert lib.knn_build_ex(ctx.handle, x.data_ptr(), n, d, k, 2, 60, 0, 0, 1, idx.data_ptr(), key.data_ptr(),
+                            ctypes.byref(opt), None) == 0
+    ctx.close()
+    held, lists = set(), []
+    for r in range(world):
+        r0, r1 = acknn.sharded.point_range(n, r, world)
+        oi, ok, fl = torch.empty_like(idx), torch.empty_like(key), torch.zeros((n, 1), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        ctx = acknn.Context(0)
+        assert lib.knn_propagate_range(ctx.handle, x.data_ptr(), n, d, k, 0, r0, r1, idx.data_ptr(), key.data_ptr(), None,
+                                       oi.data_ptr(), ok.data_ptr(), fl.data_ptr(), ctypes.byref(opt)) == 0
+        held.add(ctx.scratch_bytes)
+        lists.append((oi[r0:r1].cpu(), ok[r0:r1].cpu()))
+        ctx.close()
+    assert len(held) == 1, held
+    whole_i, whole_k = torch.empty_like(idx), torch.empty_like(key)
+    fl = torch.zeros((n, 1), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx = acknn.Context(0)
+    assert lib.knn_propagate_range(ctx.handle, x.data_ptr(), n, d, k, 0, 0, n, idx.data_ptr(), key.data_ptr(), None,
+                                   whole_i.data_ptr(), whole_k.data_ptr(), fl.data_ptr(), ctypes.byref(opt)) == 0
+    ctx.close()
+    assert torch.equal(torch.cat([i for i, _ in lists]), whole_i.cpu())
+    assert torch.equal(torch.cat([q for _, q in lists]), whole_k.cpu())
