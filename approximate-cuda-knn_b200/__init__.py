@@ -104,8 +104,10 @@ class KnnStats(ctypes.Structure):
         ("tc_group", ctypes.c_int32),
         ("sparse_dims", ctypes.c_int32),
         ("tile_pairs", ctypes.c_int32),
+        ("leaf_filtered", ctypes.c_int32),
+        ("leaf_handed", ctypes.c_int32),
         ("reserved32", ctypes.c_int32),
-        ("reserved", ctypes.c_int64 * 3),
+        ("reserved", ctypes.c_int64 * 2),
     ]
 
     def as_dict(self) -> dict:
@@ -119,6 +121,7 @@ class KnnStats(ctypes.Structure):
             "leaf_tile": self.leaf_tile, "prop_warps": self.prop_warps,
             "leaf_path": self.leaf_path, "leaf_fallback": self.leaf_fallback, "tc_group": self.tc_group,
             "sparse_dims": self.sparse_dims, "tile_pairs": self.tile_pairs,
+            "leaf_filtered": self.leaf_filtered, "leaf_handed": self.leaf_handed,
             "prop_candidates": [self.prop_candidates[i] for i in range(n)],
         }
 

@@ -527,6 +527,13 @@ bool leaf_filter_applies(const Layout& lay, int64_t n, int d, int k, int metric)
          (lay.maxleaf >= std::max(20, k + k / 2) && n * lay.maxleaf >= 800000 && d + 4 * k <= 256);
 }
 
+// Whether the filter, where it applies, takes the first tree too.  A first tree has no
+// lists to filter by, so all its pairs would survive: it takes dense tiles unless the
+// bounding pass covers every leaf (six trees, 200,000 x 128, leaf 360: 3.8 ms with the
+// first tree filtered, 5.9 without; leaf 250, where that pass does not apply: 15.8
+// against 6.5).
+bool filter_first_tree(const Layout& lay, int k) { return knn::umma_bounds_first_tree(lay.minleaf, k); }
+
 // The filter's scratch, of which a plain build has none to spare where memory is short.
 // Launches of fewer rows than 32,768 (eighth of a wave) would be slower than dense tiles.
 bool filter_scratch(knn_context* C, knn::FilterLeafArgs* f) {
@@ -539,10 +546,19 @@ bool filter_scratch(knn_context* C, knn::FilterLeafArgs* f) {
   return f->rows > 0;
 }
 
+// What the filter was given, for the statistics.
+struct FilterRun {
+  bool ran = false;
+  int first_tree = 0;
+  const unsigned long long* survivors = nullptr;  // of tree t: [t + 1]
+  unsigned long long limit = 0;
+};
+
 int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, int trees,
              const Layout& lay, int metric, const int32_t* perm, const float* norms, Lists* L,
              unsigned long long* counter, cudaStream_t st, knn::LaunchLog& log, int tile = 0,
-             cudaEvent_t* kev = nullptr, bool sparse = false, bool pairs = false, bool filter_ok = false) {
+             cudaEvent_t* kev = nullptr, bool sparse = false, bool pairs = false, bool filter_ok = false,
+             FilterRun* run = nullptr) {
   const int kw = (k + 31) / 32;
   knn::launch_init_lists(L->key[L->cur], L->id[L->cur], L->flags[L->cur], n, k, kw, st);
   log.add(2);
@@ -592,11 +608,7 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
   };
   knn::FilterLeafArgs f{};
   bool filter = filter_ok && leaf_filter_applies(lay, n, d, k, metric);
-  // A first tree has no lists to filter by, so all its pairs would survive: it takes
-  // dense tiles unless the bounding pass covers every leaf (six trees, 200,000 x 128,
-  // leaf 360: 3.8 ms with the first tree filtered, 5.9 without; leaf 250, where that
-  // pass does not apply: 15.8 against 6.5).
-  f.first_tree = filter && knn::umma_bounds_first_tree(lay.minleaf, k) ? 0 : 1;
+  f.first_tree = filter && filter_first_tree(lay, k) ? 0 : 1;
   const bool every_tree = filter && f.first_tree == 0;
   int rc = every_tree ? KNN_OK : sparse_scratch();
   if (rc) return rc;
@@ -632,6 +644,7 @@ int run_leaf(knn_context* C, const float* X, int64_t n, int d, int dpad, int k, 
   rc = a.trees > 0 ? knn::leaf_stage(a, log) : KNN_OK;
   if (rc) return fail_cuda(cudaGetLastError(), "leaf stage launch");
   if (!filter) return KNN_OK;
+  if (run) *run = {true, f.first_tree, f.survivors, knn::filter_survivor_limit(f)};
   f.dense_tree = [&](int t, const unsigned long long* survivors, unsigned long long limit) {
     knn::LeafArgs one = a;
     one.first_tree = t;
@@ -931,14 +944,17 @@ int pick_shapes(knn_context* C, const knn_options& o, bool may_tune, bool fp32_l
     sh->tc_group = std::min(sh->tc_group, lay.tc_group_max);
   }
   if (!o.autotune) return KNN_OK;
+  // no dense tile to tune where the filter takes every tree
+  const bool dense_leaf = fp32_leaf && !(filter_allowed(o) && leaf_filter_applies(lay, n, d, k, metric) &&
+                                         filter_first_tree(lay, k));
   auto it = C->tuned.find(key);
   if (it != C->tuned.end()) {
     if (!sh->leaf_tile) sh->leaf_tile = it->second.first;
     if (!sh->prop_warps) sh->prop_warps = it->second.second;
-    if (!(fp32_leaf && sh->leaf_tile == 0) && !(props > 0 && sh->prop_warps == 0)) return KNN_OK;
+    if (!(dense_leaf && sh->leaf_tile == 0) && !(props > 0 && sh->prop_warps == 0)) return KNN_OK;
   }
   if (!may_tune) return KNN_OK;
-  if (fp32_leaf && !sh->leaf_tile) {
+  if (dense_leaf && !sh->leaf_tile) {
     int rc = tune_leaf_tile(C, X, n, d, dpad, k, lay, metric, perm, norms, *L, st, sh->sparse, sh->pairs,
                             &sh->leaf_tile);
     if (rc) return rc;
@@ -1226,12 +1242,13 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
     kev = C->kernel_events(trees);
     if (!kev) return fail_cuda(cudaGetLastError(), "event creation");
   }
+  FilterRun run;
   if (tensor_leaf) {
     rc = run_leaf_umma(C, P.X, n, d, P.dpad, k, trees, lay, metric, o.precision, T.perm, norms, &L, err_flag, st,
                        log, kev, sh.tc_group);
   } else {
     rc = run_leaf(C, P.X, n, d, P.dpad, k, trees, lay, metric, T.perm, norms, &L, stats ? counters : nullptr, st,
-                  log, sh.leaf_tile, kev, sh.sparse, sh.pairs, filter_allowed(o));
+                  log, sh.leaf_tile, kev, sh.sparse, sh.pairs, filter_allowed(o), &run);
   }
   if (rc) return rc;
   if (timed) KNN_CK(cudaEventRecord(C->ev[3], st));
@@ -1302,12 +1319,19 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
     }
     stats->launches = log.count;
     stats->props_run = props;
-    stats->leaf_tile = tensor_leaf ? 128 : (sh.leaf_tile ? sh.leaf_tile : 64);
+    if (run.ran) {
+      std::vector<unsigned long long> surv(trees + 1);
+      KNN_CK(cudaMemcpy(surv.data(), run.survivors, sizeof(surv[0]) * surv.size(), cudaMemcpyDeviceToHost));
+      for (int t = run.first_tree; t < trees; ++t) ++(surv[t + 1] > run.limit ? stats->leaf_handed : stats->leaf_filtered);
+    }
+    const bool first_dense = !tensor_leaf && (!run.ran || run.first_tree > 0);  // k_leaf and k_leaf_pair ran
+    const bool dense = first_dense || stats->leaf_handed > 0;
+    stats->leaf_tile = tensor_leaf || !dense ? 128 : (sh.leaf_tile ? sh.leaf_tile : 64);
     stats->leaf_path = tensor_leaf ? o.precision : 0;
-    stats->tc_group = tensor_leaf ? std::min(std::max(sh.tc_group, 1), lay.tc_group_max) : 0;
+    stats->tc_group = tensor_leaf ? std::min(std::max(sh.tc_group, 1), lay.tc_group_max) : run.ran ? lay.tc_group_max : 0;
     stats->leaf_fallback = (o.precision != KNN_PREC_FP32 && !tensor_leaf) ? 1 : 0;
-    stats->sparse_dims = (!tensor_leaf && sh.sparse) ? 1 : 0;
-    stats->tile_pairs = (!tensor_leaf && sh.pairs) ? 1 : 0;
+    stats->sparse_dims = (first_dense && sh.sparse) ? 1 : 0;
+    stats->tile_pairs = (first_dense && sh.pairs) ? 1 : 0;
     stats->prop_warps = sh.prop_warps;
     unsigned long long host[2 + KNN_MAX_PROPS];
     KNN_CK(cudaMemcpy(host, counters, sizeof(host), cudaMemcpyDeviceToHost));

@@ -210,6 +210,8 @@ struct FilterLeafArgs {
 };
 // The bounding pass covers every leaf of at least minleaf points that is its own block.
 bool umma_bounds_first_tree(int64_t minleaf, int k);
+// A tree with more survivors than this was handed over.
+unsigned long long filter_survivor_limit(const FilterLeafArgs& a);
 bool filter_map(FilterLeafArgs* a);  // the tensor map of Xp; false where the driver refuses it
 int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log);
 size_t filter_scratch_rows(const FilterLeafArgs& a);  // from the shape fields

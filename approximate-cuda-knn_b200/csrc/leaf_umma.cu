@@ -1680,6 +1680,14 @@ size_t filter_scratch_rows(const FilterLeafArgs& a) {
 // width reach 1.25 k at every size from minleaf on if they do at 256.
 bool umma_bounds_first_tree(int64_t minleaf, int k) { return minleaf >= kPrepassMin && 8 * (k + k / 4) <= kPrepassMin; }
 
+// Data that the 16-bit rows cannot tell apart (several scales within one leaf)
+// would send most pairs down the survivors' path, at several times a dense
+// tile's cost (400,000 x 256, leaf 1,000, all pairs: 415 ms against 64), so from
+// an eighth of the pairs and 16 + k a row the dense tiles take over.
+unsigned long long filter_survivor_limit(const FilterLeafArgs& a) {
+  return (unsigned long long)a.n * (unsigned long long)(16 + a.k + a.maxleaf / 8);
+}
+
 bool filter_map(FilterLeafArgs* a) {
   CUtensorMap map;
   if (!operand_map(a->Xp, a->n, umma_row_stride(a->d), true, &map)) return false;
@@ -1730,12 +1738,8 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   t.dpad = a.dpad;
   t.metric = a.metric;
   const int64_t blocks = (a.leaves >> shape.glog) * shape.qtiles;
-  // Data that the 16-bit rows cannot tell apart (several scales within one leaf)
-  // would send most pairs down the survivors' path, at several times a dense
-  // tile's cost (400,000 x 256, leaf 1,000, all pairs: 415 ms against 64), so from
-  // an eighth of the pairs and 16 + k a row the dense tiles take over.
   cudaMemsetAsync(a.survivors, 0, sizeof(unsigned long long) * (size_t)(a.trees + 2), st);
-  t.survivor_limit = (unsigned long long)a.n * (unsigned long long)(16 + a.k + a.maxleaf / 8);
+  t.survivor_limit = filter_survivor_limit(a);
   for (int tr = a.first_tree; tr < a.trees; ++tr) {
     if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
     t.perm = a.perm + (size_t)tr * a.n;

@@ -138,18 +138,22 @@ typedef struct knn_stats {
   int64_t prop_candidates[KNN_MAX_PROPS]; /* keys evaluated per propagation iteration  */
   float ms_prop_iter[KNN_MAX_PROPS];      /* device time per propagation iteration     */
   float ms_learn;            /* learned splits: sample graph, training and embedding    */
-  int32_t leaf_tile;         /* leaf tile used: 32/64 FP32, 128 tensor-core             */
+  int32_t leaf_tile;         /* leaf tile used: 32/64 FP32, 128 tensor-core (also where
+                                the filter decided every tree of an FP32 build)       */
   int32_t prop_warps;        /* propagation warps per block used (0: the default)       */
   float ms_leaf_tiles;       /* summed device time of the leaf-tile kernel launches     */
-  int32_t leaf_path;         /* leaf stage that ran: 0 FP32 CUDA cores, 1 BF16 tensor-core
-                                tiles, 2 FP16 tensor-core tiles                        */
+  int32_t leaf_path;         /* precision of the leaf stage that ran: 0 FP32, 1 BF16
+                                tensor-core tiles, 2 FP16 tensor-core tiles            */
   int32_t leaf_fallback;     /* 1: tensor-core precision was asked for, FP32 ran        */
-  int32_t tc_group;          /* sibling leaves per tensor-core tile used (0: FP32 path) */
-  int32_t sparse_dims;       /* 1: the FP32 leaf tiles read each block's non-zero dims
+  int32_t tc_group;          /* sibling leaves per tensor-core tile used (0: no such tile) */
+  int32_t sparse_dims;       /* 1: dense FP32 leaf tiles read each block's non-zero dims
                                 (knn_build_ex; 0 from knn_build_batch)               */
-  int32_t tile_pairs;        /* 1: the FP32 leaf tiles ran as tile pairs (knn_build_ex) */
+  int32_t tile_pairs;        /* 1: dense FP32 leaf tiles ran as tile pairs (knn_build_ex) */
+  int32_t leaf_filtered;     /* trees of an FP32 build whose pairs the tensor-core filter
+                                ruled out or left to exact keys (knn_build_ex)         */
+  int32_t leaf_handed;       /* trees that it handed over to dense tiles (knn_build_ex) */
   int32_t reserved32;
-  int64_t reserved[3];
+  int64_t reserved[2];
 } knn_stats;
 
 typedef struct knn_context knn_context;
