@@ -508,7 +508,8 @@ int exact_fp64(const float* X, int64_t n, int d, int dpad, int k, int metric,
   const bool vec = (dpad & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
 #define KNN_EXACT(M, KP)                                                                                            \
   do {                                                                                                              \
-    /* also where the filter stays off: it loads the kernel, so that a warm-up call does */                          \
+    /* also where the filter stays off: with lazy loading a kernel's first use may allocate, and one small call  */ \
+    /* ahead of time is what lets knn_exact_fp64_noalloc's later ones run in a process without free memory        */ \
     cudaFuncSetAttribute(k_exact_filtered<M, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FilterSmem)); \
     if (filter) {                                                                                                   \
       k_exact_filtered<M, KP><<<grid, 256, sizeof(FilterSmem), st>>>(X, n, d, dpad, vec, k, queries, nq, norms, slice, \

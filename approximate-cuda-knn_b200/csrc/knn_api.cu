@@ -513,14 +513,14 @@ Layout single_layout(int64_t n, int depth) {
   return y;
 }
 
-// Whether the FP32 leaf stage goes through the tensor-core filter.  Six trees, dense
-// against filtered (ms): leaves of 80 points and more gain at every size (k = 8, d =
-// 64: 300 points, leaf 75, 0.44 against 0.38; 20,000, leaf 78, 1.20 against 0.84;
-// 200,000, leaf 97, 4.55 against 3.26; leaf 360, 9.7 against 3.0).  Smaller leaves
-// have little to reject, so it takes some rows to win back the launches (d = 64: 20,000 at leaf
-// 30 0.50 against 0.56, 40,000 at leaf 30 0.84 against 0.81), lists much shorter than a leaf
-// and rows short enough for a survivor's exact key to cost little more than a
-// dense tile's (200,000, leaf 49: k = 24, d = 128 4.88 against 4.62, d = 240 6.30 against 6.85).
+// Whether the FP32 leaf stage goes through the tensor-core filter: leaves of at least 80
+// points, or smaller ones of enough points in all to win back the launches, with lists much shorter
+// than a leaf and rows short enough for a survivor's exact key to cost little more than a dense
+// tile's.  Swept over 376 shapes (1,000 to 100,000 points, 16 to 256 dims, leaves of 20 to 100, k = 4
+// to 24, EUCLIDEAN and COSINE; six trees, filtered against tile pairs): nowhere slower where
+// the rule takes the filter.  It stays off the safe side of the line: 5,000 points, leaf 79
+// 0.59 to 0.72, 20,000 x 256, leaf 79 0.68 to 0.76, 100,000 x 256, leaf 25 0.73 would gain too; 20,000 x 64,
+// leaf 30 1.12, 200,000 x 240, leaf 49, k = 24 1.09 would lose.
 bool leaf_filter_applies(const Layout& lay, int64_t n, int d, int k, int metric) {
   if (metric == KNN_METRIC_TAXICAB || d > 256 || k > 32 || !lay.own_blocks || lay.ftable || !lay.tree_inv) return false;
   return lay.maxleaf >= 80 ||

@@ -216,6 +216,9 @@ bool filter_map(FilterLeafArgs* a);  // the tensor map of Xp; false where the dr
 int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log);
 size_t filter_scratch_rows(const FilterLeafArgs& a);  // from the shape fields
 
+// *out = the bits of the largest |x| over rows of dpad (a multiple of 4) floats.
+void launch_max_abs(const float* X, int64_t n, int dpad, unsigned int* out, cudaStream_t st);
+
 // 16-bit rows for the propagation's candidate filter (propagate.cu).
 inline int prop_row_stride(int d) { return (d + 7) & ~7; }
 bool prop_filter_applies(int k, int d);

@@ -1,6 +1,8 @@
 // Initial k-NN over leaf blocks on the 5th-generation tensor cores (tcgen05),
 // for EUCLIDEAN and COSINE: the mixed-precision leaf stage.
 //
+// Also the filter in front of the FP32 leaf stage (BOUND, leaf_stage_filtered below).
+//
 // Same blocks and same union-over-trees rule as the FP32 leaf stage (which
 // replaces findInitialStateOfAproximated*KNN, euclideandistancematrixgpu.cu:107-1031),
 // but every (query, candidate) key of a block comes from one BF16 GEMM tile:
@@ -21,7 +23,8 @@
 //   * an MMA thread issues tcgen05.mma.cta_group::1.kind::f16, M=128 N=64 K=16:
 //     the queries (A) stay in tensor memory for the whole block, the candidates
 //     (B) come from the ring, and QT query tiles share each candidate box; the
-//     FP32 accumulators rotate over NB 64-column buffers per query tile;
+//     FP32 accumulators rotate over NB 64-column buffers per query tile (one up to
+//     128 dims, where a tile's products wait for the last tile's to be read; two above);
 //   * four epilogue warps per query tile, one per lane quarter: a thread owns a
 //     query row.  It reads a tile's two 32-column slices with tcgen05.ld
 //     32x32b.x32, filters the products against the row's bound into survivor
@@ -1318,15 +1321,6 @@ __global__ void k_inverse_order(const int32_t* __restrict__ order, int64_t n, in
     inv[order[i]] = (int32_t)i;
 }
 
-// Largest |x| over the rows (non-negative floats order as their bit patterns).
-__global__ void k_max_abs(const float* __restrict__ X, int64_t count, unsigned int* __restrict__ out) {
-  float m = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf(X[i]));
-  m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
-}
-
 __device__ __forceinline__ uint16_t to_operand(float v, bool f16) {
   return f16 ? __half_as_ushort(__float2half_rn(v)) : __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
@@ -1583,9 +1577,7 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
   uint16_t* Xb = static_cast<uint16_t*>(a.Xb);
   // operand copy (FP16 EUCLIDEAN: the largest |x| first, for the row scale)
   if (a.f16 && a.metric == KNN_METRIC_EUCLIDEAN) {
-    cudaMemsetAsync(a.maxabs, 0, sizeof(unsigned int), st);
-    const int64_t cnt = a.n * (int64_t)a.dpad;
-    k_max_abs<<<(unsigned)std::min<int64_t>((cnt + 255) / 256, 148 * 8), 256, 0, st>>>(a.X, cnt, a.maxabs);
+    launch_max_abs(a.X, a.n, a.dpad, a.maxabs, st);
     log.add();
   }
   const int ldr = umma_row_stride(a.d);
@@ -1703,9 +1695,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   const TcShape shape = tc_shape(a.d, a.maxleaf, a.tc_group);
   const int ldr = umma_row_stride(a.d);
   if (a.metric == KNN_METRIC_EUCLIDEAN) {
-    cudaMemsetAsync(a.maxabs, 0, sizeof(unsigned int), st);
-    const int64_t cnt = a.n * (int64_t)a.dpad;
-    k_max_abs<<<(unsigned)std::min<int64_t>((cnt + 255) / 256, 148 * 8), 256, 0, st>>>(a.X, cnt, a.maxabs);
+    launch_max_abs(a.X, a.n, a.dpad, a.maxabs, st);
     log.add();
   }
   CUtensorMap map;

@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kPropMaxWarps * 32) k_propagate(
 constexpr float kDeltaUp = 1.0f + 1.0f / 1024.0f;  // delta is itself computed in FP32
 
 // Largest |x| over the rows (non-negative floats order as their bit patterns).
-__global__ void __launch_bounds__(256) k_prop_max_abs(const float4* __restrict__ X, int64_t count,
+__global__ void __launch_bounds__(256) k_max_abs(const float4* __restrict__ X, int64_t count,
                                                       unsigned int* __restrict__ out) {
   float m = 0.f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
@@ -778,14 +778,18 @@ bool prop_filter_pays(int k, int d, int metric, bool half) {
   return d <= 256 ? idle < 1.33 || k < 6 : idle < 1.45;
 }
 
+void launch_max_abs(const float* X, int64_t n, int dpad, unsigned int* out, cudaStream_t st) {
+  cudaMemsetAsync(out, 0, sizeof(unsigned int), st);
+  const int64_t quads = n * (int64_t)(dpad / 4);
+  k_max_abs<<<(unsigned)std::min<int64_t>((quads + 255) / 256, 148 * 8), 256, 0, st>>>(reinterpret_cast<const float4*>(X),
+                                                                                       quads, out);
+}
+
 int prop_prepare(const PropPrep& a, LaunchLog& log) {
   const int ldh = prop_row_stride(a.d);
   __half* H = static_cast<__half*>(a.H);
   if (a.metric != KNN_METRIC_COSINE) {
-    cudaMemsetAsync(a.maxabs, 0, sizeof(unsigned int), a.stream);
-    const int64_t quads = a.n * (int64_t)(a.dpad / 4);
-    k_prop_max_abs<<<(unsigned)std::min<int64_t>((quads + 255) / 256, 148 * 8), 256, 0, a.stream>>>(
-        reinterpret_cast<const float4*>(a.X), quads, a.maxabs);
+    launch_max_abs(a.X, a.n, a.dpad, a.maxabs, a.stream);
     log.add();
   }
   const unsigned grid = (unsigned)((a.n + 7) / 8);
