@@ -82,10 +82,10 @@ def measured_peaks() -> tuple[float, str]:
 
 def profiled_traffic(summary: str, config: dict, n: int):
     """DRAM bytes per launch from a committed ncu summary under profiles/: the
-    line `traffic_bytes_per_launch: B n=N d=.. k=.. trees=.. leaf=..` gives the
-    mean per launch on N points; it is scaled to n (a launch's traffic grows
-    with the points it processes).  (None, reason) when the summary is absent
-    or was taken on another configuration."""
+    line `traffic_bytes_per_launch: B n=N d=.. k=.. trees=.. leaf=.. kernels=..`
+    gives the mean per tree on N points of the named kernels; it is scaled to n
+    (the traffic grows with the points).  (None, reason) when the summary is
+    absent or was taken on another configuration or other kernels."""
     import re
 
     path = ROOT / "profiles" / summary
@@ -98,8 +98,8 @@ def profiled_traffic(summary: str, config: dict, n: int):
     if any(str(config[key]) != fields.get(key) for key in config):
         return None, f"profiles/{summary} was taken on another configuration ({m.group(3)})"
     b, pn = int(m.group(1)), int(m.group(2))
-    return b * n / pn, (f"ncu dram__bytes_read.sum + dram__bytes_write.sum per launch, mean over a build's "
-                        f"launches at {pn:,} points (profiles/{summary}), scaled to {n:,} points")
+    return b * n / pn, (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of a tree's tile and merge kernels, mean over a "
+                        f"build's trees at {pn:,} points (profiles/{summary}), scaled to {n:,} points")
 
 
 def measured_tensor_peak() -> tuple[float, str]:
@@ -416,20 +416,21 @@ def run_ours(args, w):
     dom = max(cand, key=lambda kname: cand[kname][0])
     dms, dbytes, dlaunch = cand[dom]
     achieved = dbytes / (dms / 1e3) / 1e9
-    # DRAM bytes (read + write) per k_leaf_tc launch from the committed ncu
-    # summary of this kernel on a smaller case of the same configuration,
-    # scaled by the points a launch processes
+    # DRAM bytes (read + write) of a tree's k_leaf_tc and k_leaf_tc_merge launches
+    # from the committed ncu summary of these kernels on a smaller case of the same
+    # configuration, scaled by the points
     traffic, traffic_src = None, None
     if dom == "leaf_tc":
         traffic, traffic_src = profiled_traffic("k_leaf_tc_integer_mixture_500k.md",
-                                                dict(d=d, k=k, trees=T, leaf=head["leaf"]), n)
+                                                dict(d=d, k=k, trees=T, leaf=head["leaf"],
+                                                     kernels="k_leaf_tc+k_leaf_tc_merge"), n)
     hbm_view = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                 "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                 "traffic_source": traffic_src,
                 "peak_source": peak_kind,
                 "algorithmic_bytes_per_launch": dbytes / dlaunch,
                 "mean_launch_ms": dms / dlaunch,
-                "mean_launch_source": "CUDA events around each k_leaf_tc launch of the last timed step"
+                "mean_launch_source": "CUDA events around each tree's tile and merge kernels in the last timed step"
                 if dom == "leaf_tc" and leaf_kernel_ms > 0 else "stage time / launches"}
     roofline = hbm_view
     if dom == "leaf_tc":
