@@ -106,7 +106,7 @@ class KnnStats(ctypes.Structure):
         ("tile_pairs", ctypes.c_int32),
         ("leaf_filtered", ctypes.c_int32),
         ("leaf_handed", ctypes.c_int32),
-        ("reserved32", ctypes.c_int32),
+        ("prop_filtered", ctypes.c_int32),
         ("reserved", ctypes.c_int64 * 2),
     ]
 
@@ -122,6 +122,7 @@ class KnnStats(ctypes.Structure):
             "leaf_path": self.leaf_path, "leaf_fallback": self.leaf_fallback, "tc_group": self.tc_group,
             "sparse_dims": self.sparse_dims, "tile_pairs": self.tile_pairs,
             "leaf_filtered": self.leaf_filtered, "leaf_handed": self.leaf_handed,
+            "prop_filtered": self.prop_filtered,
             "prop_candidates": [self.prop_candidates[i] for i in range(n)],
         }
 

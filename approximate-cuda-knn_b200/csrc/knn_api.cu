@@ -1333,6 +1333,7 @@ int build_impl(knn_context* C, const void* points, int64_t n, int32_t d, int32_t
     stats->sparse_dims = (first_dense && sh.sparse) ? 1 : 0;
     stats->tile_pairs = (first_dense && sh.pairs) ? 1 : 0;
     stats->prop_warps = sh.prop_warps;
+    stats->prop_filtered = F.H ? 1 : 0;
     unsigned long long host[2 + KNN_MAX_PROPS];
     KNN_CK(cudaMemcpy(host, counters, sizeof(host), cudaMemcpyDeviceToHost));
     stats->leaf_pairs = (int64_t)host[0];

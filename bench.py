@@ -406,7 +406,8 @@ def run_ours(args, w):
     T, L, P = head["trees"], stages["depth"], head["props"]
     s = 4
     kq = min(32, 2 * k)
-    prop_bytes = sum(n * (k * k * 4 + 2 * k * 8) + c * d * s for c in stages["prop_candidates"])
+    ps = 2 if stages["prop_filtered"] else s  # bytes of a candidate row's element
+    prop_bytes = sum(n * (k * k * 4 + 2 * k * 8) + c * d * ps for c in stages["prop_candidates"])
     # tensor-core leaf stage: the BF16 rows (d*2 B) and each point's kq-entry list per tree
     leaf_bytes = T * (n * d * 2 + n * kq * 8 * 2)
     tree_bytes = T * L * (n * d * s + 16 * n)
@@ -734,16 +735,18 @@ PATH_OPTIONS = {
 }
 
 
-def prop_roofline(n, d, k, s, cands, ms_prop, peak):
+def prop_roofline(n, d, k, s, cands, ms_prop, peak, filtered):
     """Propagation against HBM: algorithmic bytes P N (k^2 4 + 2k 8) + sum over
-    iterations of c-bar N d s (c-bar N = the keys evaluated in that iteration,
-    each reading one candidate row of d elements of s bytes), over the
-    propagation time."""
+    iterations of c-bar N d s (c-bar N = the candidates of that iteration, each
+    reading one row of d elements of s bytes, of 2 where 16-bit rows rule most of
+    them out), over the propagation time."""
+    if filtered:
+        s = 2
     if not cands or ms_prop <= 0:
         return None
     by = sum(n * (k * k * 4 + 2 * k * 8) + c * d * s for c in cands)
     ach = by / (ms_prop / 1e3) / 1e9
-    return {"bound": "hbm", "kernel": "k_propagate", "algorithmic_bytes": by, "ms": ms_prop,
+    return {"bound": "hbm", "kernel": "k_propagate_filtered" if filtered else "k_propagate", "algorithmic_bytes": by, "ms": ms_prop,
             "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
             "c_bar": [c / n for c in cands]}
 
@@ -817,7 +820,7 @@ def run_config(args):
                      "sparse_dims": sd["sparse_dims"],
                      "stages_ms": {kk: sd[kk] for kk in ("ms_learn", "ms_trees", "ms_leaf", "ms_propagate")},
                      "propagate_roofline": prop_roofline(n, d, k, s_bytes, sd["prop_candidates"],
-                                                         sd["ms_propagate"], peak)}
+                                                         sd["ms_propagate"], peak, sd["prop_filtered"])}
     plain = res.get("plain_fp32@target")
     ratios = {}
     if plain:

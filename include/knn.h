@@ -135,7 +135,7 @@ typedef struct knn_stats {
   int32_t launches;          /* kernels launched by the call                           */
   int32_t props_run;         /* propagation iterations run                             */
   int64_t leaf_pairs;        /* (query, candidate) keys evaluated by the leaf stage     */
-  int64_t prop_candidates[KNN_MAX_PROPS]; /* keys evaluated per propagation iteration  */
+  int64_t prop_candidates[KNN_MAX_PROPS]; /* candidates considered per propagation iteration */
   float ms_prop_iter[KNN_MAX_PROPS];      /* device time per propagation iteration     */
   float ms_learn;            /* learned splits: sample graph, training and embedding    */
   int32_t leaf_tile;         /* leaf tile used: 32/64 FP32, 128 tensor-core (also where
@@ -152,7 +152,9 @@ typedef struct knn_stats {
   int32_t leaf_filtered;     /* trees of an FP32 build whose pairs the tensor-core filter
                                 ruled out or left to exact keys (knn_build_ex)         */
   int32_t leaf_handed;       /* trees that it handed over to dense tiles (knn_build_ex) */
-  int32_t reserved32;
+  int32_t prop_filtered;     /* 1: propagation ruled candidates out by their 16-bit rows,
+                                exact keys for the rest; 0: a key for each candidate
+                                (knn_build_ex)                                       */
   int64_t reserved[2];
 } knn_stats;
 

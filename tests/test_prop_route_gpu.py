@@ -61,3 +61,13 @@ def test_ranges_of_a_step_take_one_route(world):
     ctx.close()
     assert torch.equal(torch.cat([i for i, _ in lists]), whole_i.cpu())
     assert torch.equal(torch.cat([q for _, q in lists]), whole_k.cpu())
+
+
+def test_statistics_name_the_route():
+    acknn = load_package()
+    for d, k, metric, dtype, want in ((64, 16, 0, np.float32, 1), (300, 8, 0, np.float32, 0), (300, 8, 2, np.float32, 0),
+                                      (200, 8, 0, np.float32, 1), (200, 8, 0, np.float16, 0), (8, 5, 1, np.float32, 0),
+                                      (1030, 8, 0, np.float32, 0)):
+        x = acknn.workloads.gaussian_mixture(600, d, 4, seed=d).astype(dtype)
+        assert acknn.knn_build(x, k, 2, 30, 1, metric, stats=True)[2]["prop_filtered"] == want
+        assert acknn.knn_build(x, k, 2, 30, 0, metric, stats=True)[2]["prop_filtered"] == 0
