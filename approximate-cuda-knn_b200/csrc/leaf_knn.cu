@@ -879,8 +879,9 @@ namespace {
 //   leaves of 586 (2 blocks):  whole 24.7 / 26.7, query tiles 25.9 / 21.9, k_leaf 36.2 / 32.5,
 //                              k_leaf_pair 28.2 / 26.3
 // Clusters of 2 to 8 blocks per leaf, a barrier between the rounds of k_leaf_pair: 20.5 and 32.4.
+constexpr int kWholeLists = 76 * 1024;
 bool handed_whole(int metric, int64_t leaves, int64_t maxleaf, int k) {
-  return leaves >= 2 * 148 && maxleaf * k * 8 <= (metric == KNN_METRIC_EUCLIDEAN ? 76 : 39) * 1024;
+  return leaves >= 2 * 148 && maxleaf * k * 8 <= (metric == KNN_METRIC_EUCLIDEAN ? kWholeLists : 39 * 1024);
 }
 
 template <int METRIC, int TILE, bool WHOLE>
@@ -888,7 +889,9 @@ void launch_handed(const LeafArgs& a) {
   const int rows = WHOLE ? (int)a.maxleaf : TILE;
   const int64_t tiles = WHOLE ? 1 : (a.maxleaf + TILE - 1) / TILE;
   const int smem = rows * a.k * 8;
-  cudaFuncSetAttribute(k_leaf_handed<METRIC, TILE, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // the attribute is the process's: one value, whatever shapes other threads launch
+  cudaFuncSetAttribute(k_leaf_handed<METRIC, TILE, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       WHOLE ? kWholeLists : TILE * 32 * 8);
   // most of these launches return at once: no more blocks than fill the chip twice
   const unsigned grid = (unsigned)std::min<int64_t>(a.leaves * tiles, 148 * 8);
   k_leaf_handed<METRIC, TILE, WHOLE><<<grid, 256, smem, a.stream>>>(

@@ -272,7 +272,6 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 // Lists and candidates are (ordered key, id) pairs compared as one 64-bit
 // number: ordered keys are the FP32 keys mapped to integers of the same order.
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
-constexpr uint32_t kInfKey = 0xFF800000u;  // +inf
 __device__ __forceinline__ float from_orderable(uint32_t o) {
   return __uint_as_float((o & 0x80000000u) ? (o ^ 0x80000000u) : ~o);
 }
@@ -518,11 +517,8 @@ __device__ __forceinline__ float merge_survivors(uint32_t* akey, uint32_t* aid, 
           }
           const float dot = __uint_as_float(v.x);
           const uint32_t p = v.y;
-          // a key that is not a number (rows with infinite values) goes last: its sign bit, which
-          // would rank it, depends on how the expression was compiled
-          const float key = METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(xn, np[p]))
-                                                           : __fsub_rn(1.f, dot);
-          ck[i] = key < __int_as_float(0x7F800000) ? orderable(key) : kInfKey;
+          ck[i] = orderable(METRIC == KNN_METRIC_EUCLIDEAN ? __fmaf_rn(-2.f, dot, __fadd_rn(xn, np[p]))
+                                                           : __fsub_rn(1.f, dot));
           ci[i] = (uint32_t)perm[p];
         }
       }
@@ -1334,7 +1330,9 @@ __device__ __forceinline__ float from_operand(uint16_t b, bool f16) {
 // of two 2^e that brings the largest |x| (maxabs) into [2^14, 2^15), inside
 // the FP16 range: a power-of-two scale is exact, scales every key of the tile
 // stage by the same 2^2e and so keeps its ranking (the re-rank uses X).  With perm,
-// output row i is row perm[i].
+// output row i is row perm[i].  A row with infinite values or NaN becomes a zero row with
+// an infinite norm (COSINE: a key of 1): products with it would give keys of the form
+// inf - inf, whose order is not defined, and it is no finite row's neighbour.
 __global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int dpad, int ldr, int metric, bool f16,
                              const unsigned int* __restrict__ maxabs, const float* __restrict__ norms,
                              const int32_t* __restrict__ perm, uint16_t* __restrict__ Xb, float* __restrict__ norms2) {
@@ -1357,8 +1355,10 @@ __global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int 
     scale = ldexpf(1.f, e);
   }
   float s = 0.f;
+  bool finite = true;
   for (int c = lane; c < ldr; c += 32) {
     const float v = c < d ? X[(size_t)row * dpad + c] : 0.f;
+    finite &= fabsf(v) < __int_as_float(0x7F800000);
     const uint16_t b = to_operand(__fmul_rn(v, scale), f16);
     Xb[(size_t)out * ldr + c] = b;
     const float f = from_operand(b, f16);
@@ -1366,6 +1366,10 @@ __global__ void k_to_operand(const float* __restrict__ X, int64_t n, int d, int 
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xFFFFFFFFu, s, off));
+  if (!__all_sync(0xFFFFFFFFu, finite)) {
+    for (int c = lane; c < ldr; c += 32) Xb[(size_t)out * ldr + c] = 0;
+    s = __int_as_float(0x7F800000);
+  }
   if (lane == 0) norms2[out] = s;
 }
 
@@ -1649,13 +1653,16 @@ int leaf_stage_umma(const UmmaLeafArgs& a, LaunchLog& log) {
       launch_tc_tree<KNN_METRIC_COSINE, false>(tr == 0, pre, qt, nch, map, t, blocks, a.rows, nullptr, nullptr, st, log);
     if (a.kev) cudaEventRecord(a.kev[2 * tr + 1], st);
   }
-  const size_t rsm = (size_t)8 * (a.dpad + 32 * 64 + 32) * sizeof(float);
+  // shared memory of k_rerank's eight warps; the attribute is the process's, so one value for all dims
+  auto rerank_smem = [](int dpad) { return (size_t)8 * (dpad + 32 * 64 + 32) * sizeof(float); };
+  const size_t rsm = rerank_smem(a.dpad);
+  const int rsm_max = (int)rerank_smem(4 * kKC);
   const unsigned rgrid = (unsigned)((a.n + 7) / 8);
   if (a.metric == KNN_METRIC_EUCLIDEAN) {
-    cudaFuncSetAttribute(k_rerank<KNN_METRIC_EUCLIDEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
+    cudaFuncSetAttribute(k_rerank<KNN_METRIC_EUCLIDEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm_max);
     k_rerank<KNN_METRIC_EUCLIDEAN><<<rgrid, 256, rsm, st>>>(a.X, a.n, a.d, a.dpad, a.k, a.kq, a.norms, a.aid, a.rkey, a.rid);
   } else {
-    cudaFuncSetAttribute(k_rerank<KNN_METRIC_COSINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm);
+    cudaFuncSetAttribute(k_rerank<KNN_METRIC_COSINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm_max);
     k_rerank<KNN_METRIC_COSINE><<<rgrid, 256, rsm, st>>>(a.X, a.n, a.d, a.dpad, a.k, a.kq, a.norms, a.aid, a.rkey, a.rid);
   }
   log.add();

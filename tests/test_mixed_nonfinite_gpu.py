@@ -1,4 +1,4 @@
-"""Rows with infinite values in a tensor-core build: their approximate keys are not numbers and must not displace the
+"""Rows with infinite values in a tensor-core build: their approximate keys have no order and must not displace the
 neighbours of the other rows.  On integer rows every product and sum of the tiles is exact, so wherever a plain FP32
 build (the same trees) lists finite distances only, the mixed build lists the same."""
 from __future__ import annotations
