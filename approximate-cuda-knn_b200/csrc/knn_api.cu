@@ -540,7 +540,7 @@ bool filter_scratch(knn_context* C, knn::FilterLeafArgs* f) {
   const size_t rows = knn::filter_scratch_rows(*f);
   if (!C->spare("Xp", (size_t)f->n * knn::umma_row_stride(f->d) * 2, &f->Xp) || !C->spare("norms_perm", (size_t)f->n, &f->np) ||
       !C->spare("delta_perm", (size_t)f->n, &f->dp) || !C->spare("maxabs", 1, &f->maxabs) ||
-      !C->spare("leaf_survivors", (size_t)f->trees + 2, &f->survivors))
+      !C->spare("leaf_survivors", knn::filter_counters(f->trees), &f->survivors))
     return false;
   f->rows = (int64_t)C->spare_survivors(rows, std::min<size_t>(rows, 1 << 15), &f->surv, &f->count);
   return f->rows > 0;

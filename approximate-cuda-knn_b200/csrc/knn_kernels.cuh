@@ -198,7 +198,8 @@ struct FilterLeafArgs {
   void* surv;               // [rows][umma_row_scratch_bytes()] scratch
   uint32_t* count;          // [rows] scratch
   unsigned int* maxabs;
-  // [trees + 2] scratch: a zero, each tree's survivors, and the words of waits that gave up
+  // [filter_counters(trees)] scratch: a zero, each tree's survivors, and, kFilterErrGap
+  // further on, the words of waits that gave up
   unsigned long long* survivors;
   // launches tree t's dense tiles, which run if *survivors > limit
   std::function<int(int t, const unsigned long long* survivors, unsigned long long limit)> dense_tree;
@@ -208,6 +209,11 @@ struct FilterLeafArgs {
   cudaEvent_t* kev;
   cudaStream_t stream;
 };
+// Every block reads the words of waits that gave up, every tile adds to its tree's
+// survivors: on one cache line the reads queue behind the sums (k_leaf_tc_exact, COSINE,
+// 19,683 x 134, leaf 663: 25.9 us a tree on one line, 24.6 with 256 bytes between them).
+constexpr int kFilterErrGap = 32;
+inline size_t filter_counters(int trees) { return (size_t)trees + 1 + kFilterErrGap + 1; }
 // The bounding pass covers every leaf of at least minleaf points that is its own block.
 bool umma_bounds_first_tree(int64_t minleaf, int k);
 // A tree with more survivors than this was handed over.

@@ -1713,7 +1713,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   t.dp = a.dp;
   t.segs = a.segs;
   t.aid = a.rid;
-  t.err = reinterpret_cast<int*>(a.survivors + a.trees + 1);
+  t.err = reinterpret_cast<int*>(a.survivors + a.trees + 1 + kFilterErrGap);
   t.n = a.n;
   t.idesc = idesc_for(true);
   t.ldr = ldr;
@@ -1735,7 +1735,7 @@ int leaf_stage_filtered(const FilterLeafArgs& a, LaunchLog& log) {
   t.dpad = a.dpad;
   t.metric = a.metric;
   const int64_t blocks = (a.leaves >> shape.glog) * shape.qtiles;
-  cudaMemsetAsync(a.survivors, 0, sizeof(unsigned long long) * (size_t)(a.trees + 2), st);
+  cudaMemsetAsync(a.survivors, 0, sizeof(unsigned long long) * filter_counters(a.trees), st);
   t.survivor_limit = filter_survivor_limit(a);
   for (int tr = a.first_tree; tr < a.trees; ++tr) {
     if (a.kev) cudaEventRecord(a.kev[2 * tr], st);
